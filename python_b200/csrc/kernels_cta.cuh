@@ -71,7 +71,9 @@ struct CtaShape {
   static constexpr int off_V = off_Mm + P * MS;
   static constexpr int off_r = off_V + B * P;
   static constexpr int off_pb = off_r + B; // pivot-row exchange of a multi-warp panel
-  static constexpr int n_dbl = off_pb + B + 2;
+  // solves: the right-hand side rides along by row, its pivot values of a panel beside it
+  static constexpr int off_rhs = off_pb + B + 2;
+  static constexpr int n_dbl = off_rhs + (KIND == kSolve ? P + B : 0);
   static constexpr int n_int = 2 * P + 4 + 4 * PW;
   static constexpr size_t dyn_smem = size_t(n_dbl) * 8 + size_t(n_int) * 4;
   static constexpr int by_smem = int(kSmemPerSm / (dyn_smem + 1024));
@@ -85,6 +87,7 @@ struct CtaShape {
   static_assert(P % TGR == 0 && RB % RG == 0 && CB % CC == 0, "whole update tiles");
   static_assert(PW >= 1 && PW <= NW, "panel warps are warps of the CTA");
   static_assert(dyn_smem <= 232448, "one CTA's shared memory");
+  static_assert((P + 31) / 32 * 32 * MS <= P * MS + 4 * P, "the residual check's tiles end below the solution");
 };
 
 template <int KIND, int P, int NT, int RG, int CC, int PW, bool GM, int MINB>
@@ -102,7 +105,9 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
   double* pivbuf = dsm + Sh::off_pb;       // [B+1] pivot row and its reciprocal (PW > 1)
   int* ps_s = reinterpret_cast<int*>(dsm + Sh::n_dbl);   // [P] position of each row
   int* perm = ps_s + P;                    // [P] row at each position
-  int* flags = perm + P;                   // [0] singular, [1] an infinite pivot
+  int* flags = perm + P;                   // [0] singular, [1] an infinite pivot, [2] first failing row of a solve
+  double* rhs = dsm + Sh::off_rhs;         // solves: [P] right-hand side by row, [B] the panel's pivot values
+  double* vrhs = rhs + P;
   unsigned* cand = reinterpret_cast<unsigned*>(flags + 4);   // [PW][4] per-warp pivot candidates
 
   const int t = threadIdx.x;
@@ -132,7 +137,10 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
     if (t == 0) {
       flags[0] = 0;
       flags[1] = 0;
+      flags[2] = 0x7fffffff;
     }
+    if (KIND == kSolve)
+      for (int r = t; r < n; r += NT) rhs[r] = bv.b[bv.offv[s] + r];
     if (!GM) cp_async_wait_all();
     __syncthreads();
 
@@ -347,6 +355,31 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
       if (flags[0]) { singular = true; break; }
 
       // ---- 2. the panel's pivot rows at their own step, one thread per column
+      // (a solve's right-hand side is one more column: the forward sweep of
+      // LU_svx subtracts l_ij y_j from b_i with j ascending, as here)
+      if (KIND == kSolve && t == NT - 1) {
+        int q[B];
+        double v[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+          q[k] = perm[j0 + k];
+          v[k] = (k < nb) ? rhs[q[k]] : 0.0;
+        }
+#pragma unroll
+        for (int k = 1; k < B; ++k) {
+          double ml[B];
+#pragma unroll
+          for (int k2 = 0; k2 < k; ++k2) ml[k2] = Mm[q[k] * MS + k2];
+#pragma unroll
+          for (int k2 = 0; k2 < k; ++k2)
+            if (k < nb) v[k] = sub_rn(v[k], mul_rn(ml[k2], v[k2]));
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+          vrhs[k] = v[k];
+          if (k < nb) rhs[q[k]] = v[k];
+        }
+      }
       for (int c = t; c < P; c += NT) {
         if (!((c < j0 || c >= j0 + B) && (KIND == kInvert || c >= j0 + B))) continue;
         if constexpr (!GM) {
@@ -430,6 +463,15 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
       __syncthreads();
 
       // ---- 3. update of every other row outside the panel ----------------------
+      if (KIND == kSolve) {
+        for (int r = t; r < n; r += NT) {
+          if (ps_s[r] < j0 + B) continue;
+          double v = rhs[r];
+#pragma unroll
+          for (int k = 0; k < B; ++k) v = sub_rn(v, mul_rn(Mm[r * MS + k], vrhs[k]));
+          rhs[r] = v;
+        }
+      }
       if (!GM) {
         // Shared memory: column by column.  The panel's own columns are
         // skipped, a solve skips its L columns too, and the inverse's columns
@@ -573,58 +615,121 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
         if (bv.diag) bv.diag[s] = kDiagExact;
       }
     } else {
-      // LU_svx (lu.c:324-360): permute b, unit-lower then upper sweep, each entry
-      // in GSL's order; row q of the factors is row perm[q] of M
-      double* vec = Vs;                    // [P]
-      double* xs = Vs + P;                 // [P]
+      // The upper sweep of LU_svx (lu.c:324-360; the lower one rode along with
+      // the factorisation): x_i = (y_i - U_i,i+1 x_i+1 - U_i,i+2 x_i+2 - ...) /
+      // U_ii.  Each sum starts with the x just found, so GSL's order is one
+      // chain of n^2 / 2 dependent subtractions; everything else is kept off it.
+      // Warp 0 holds row i's products U_ik x_k, k >= i + 2, in shared memory
+      // (formed by its 32 lanes while row i + 1's chain ran; zeros pad both
+      // ends of the range, and u - 0 = u), every lane runs the chain from
+      // broadcast 16-byte loads, and row i - 1's entries are on their way
+      // meanwhile.  It was one lane walking U, each step waiting on its load:
+      // n = 204 alone on an SM took 1.1 ms in all, and 4,096 systems of orders
+      // 33-200 8.02 ms (4.99 ms now).
+      double* Pb = Vs;                     // [P + 8] products of the current row
+      double* xs = Vs + 4 * P;             // [P] solution, clear of the check's tiles below
+      const int64_t ov = bv.offv[s];
       if (wid == 0) {
-        const int64_t ov = bv.offv[s];
-        for (int i = wl; i < n; i += 32) vec[i] = bv.b[ov + perm[i]];
+        const int r = perm[n - 1];
+        if (wl < 8) Pb[(n & ~7) + wl] = 0.0;
         __syncwarp();
-        for (int j = 0; j < n; ++j) {
-          const double yj = vec[j];
-          for (int i = j + 1 + wl; i < n; i += 32) {
-            const int r = perm[i];
-            vec[i] = sub_rn(vec[i], mul_rn(M[r * P + (j ^ cta_swz(r))], yj));
+        double y = rhs[r], d = M[r * P + ((n - 1) ^ cta_swz(r))], e = 0.0, xp = 0.0;
+        for (int i = n - 1; i >= 0; --i) {
+          const int ip = (i > 0) ? i - 1 : 0;
+          const int rn = perm[ip], swn = cta_swz(rn);
+          const double* Un = M + rn * P;
+          const double yn = rhs[rn], dn = Un[ip ^ swn], en = Un[i ^ swn];
+          double u = y;
+          if (i + 1 < n) u = sub_rn(u, mul_rn(e, xp));
+          // in pieces of 256 columns: row i - 1's entries loaded, row i's chain, then
+          // row i - 1's products over the ones just used
+          const int kn = i + 1;            // first product of row i - 1
+          for (int kc = kn & ~7; kc < n; kc += 256) {
+            double un[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+              const int k = kc + wl + 32 * m;
+              un[m] = (k >= kn && k < n) ? Un[k ^ swn] : 0.0;
+            }
+            const int ke = min(n, kc + 256);
+            for (int k = max(kc, (i + 2) & ~7); k < ke; k += 8) {
+              const double2* p2 = reinterpret_cast<const double2*>(Pb + k);
+              const double2 p0 = p2[0], p1 = p2[1], p3 = p2[2], p4 = p2[3];
+              u = sub_rn(u, p0.x);
+              u = sub_rn(u, p0.y);
+              u = sub_rn(u, p1.x);
+              u = sub_rn(u, p1.y);
+              u = sub_rn(u, p3.x);
+              u = sub_rn(u, p3.y);
+              u = sub_rn(u, p4.x);
+              u = sub_rn(u, p4.y);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+              const int k = kc + wl + 32 * m;
+              if (k < ((n + 7) & ~7)) Pb[k] = (k >= kn && k < n) ? mul_rn(un[m], xs[k]) : 0.0;
+            }
           }
+          xp = div_rn(u, d);
+          if (wl == 0) xs[i] = xp;
           __syncwarp();
+          y = yn;
+          d = dn;
+          e = en;
         }
-        if (wl == 0) {
-          for (int i = n - 1; i >= 0; --i) {
-            const int r = perm[i], sw = cta_swz(r);
-            double u = vec[i];
-            for (int k = i + 1; k < n; ++k) u = sub_rn(u, mul_rn(M[r * P + (k ^ sw)], xs[k]));
-            xs[i] = div_rn(u, M[r * P + (i ^ sw)]);
+        for (int i = wl; i < n; i += 32) bv.out[ov + i] = xs[i];
+      }
+      __syncthreads();
+      // residual check on the original A (matrix_cpu.c:155-187), first failing
+      // row decides: a warp per 32 rows, A read in coalesced 32 x 32 pieces
+      // whose products reach the lane of their row through 32 x 8 tiles in the
+      // multiplier panel, added there in ascending k
+      for (int rb = wid; 32 * rb < n; rb += NW) {
+        double* tl = Mm + wid * (32 * MS);   // the last one may reach into Vs, below xs
+        const int i = 32 * rb + wl;
+        const int rr = wl >> 3, cc = wl & 7;
+        double acc = 0.0;
+        for (int c0 = 0; c0 < n; c0 += 32) {
+          double v[4][8];
+#pragma unroll
+          for (int w = 0; w < 4; ++w)
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+              const int row = 32 * rb + 4 * m + rr, col = c0 + 8 * w + cc;
+              v[w][m] = (row < n && col < n) ? __ldg(Ag + int64_t(row) * n + col) : 0.0;
+            }
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const int col = c0 + 8 * w + cc;
+            const double xc = (col < n) ? xs[col] : 0.0;
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 8; ++m) tl[(4 * m + rr) * MS + cc] = mul_rn(v[w][m], xc);
+            __syncwarp();
+            const int ce = min(8, n - c0 - 8 * w);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (k < ce) acc = add_rn(acc, tl[wl * MS + k]);
           }
         }
-        __syncwarp();
-        // residual check on the original A (matrix_cpu.c:155-187), first failing row decides
-        int first = 0x7fffffff, fcode = 0;
-        for (int i = wl; i < n; i += 32) {
-          double acc = 0.0;
-          const double* __restrict__ arow = Ag + int64_t(i) * n;
-          for (int k = 0; k < n; ++k) acc = add_rn(acc, mul_rn(arow[k], xs[k]));
-          const double y = add_rn(0.0, acc);
+        if (i < n) {
+          const double yv = add_rn(0.0, acc);
           const double bi = bv.b[ov + i];
           int code = 0;
           if (bi > 0.0) {
-            if (fabs(div_rn(sub_rn(y, bi), y)) > kResidEps) code = kResidRel;
-          } else if (fabs(sub_rn(y, bi)) > kResidEps) {
+            if (fabs(div_rn(sub_rn(yv, bi), yv)) > kResidEps) code = kResidRel;
+          } else if (fabs(sub_rn(yv, bi)) > kResidEps) {
             code = kResidAbs;
           }
-          if (code && i < first) { first = i; fcode = code; }
+          if (code) atomicMin(&flags[2], 4 * i + code);
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          const int of = __shfl_xor_sync(FULL, first, off);
-          const int oc = __shfl_xor_sync(FULL, fcode, off);
-          if (of < first) { first = of; fcode = oc; }
-        }
-        for (int i = wl; i < n; i += 32) bv.out[ov + i] = xs[i];
-        if (wl == 0) {
-          bv.status[s] = fcode;
-          if (bv.diag) bv.diag[s] = kDiagExact;
-        }
+        __syncwarp();
+      }
+      __syncthreads();
+      if (t == 0) {
+        bv.status[s] = (flags[2] == 0x7fffffff) ? kOk : (flags[2] & 3);
+        if (bv.diag) bv.diag[s] = kDiagExact;
       }
     }
     __syncthreads();
