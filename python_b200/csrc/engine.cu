@@ -1088,9 +1088,11 @@ static int run_matom_sample(int nq, int nsys, const int* n, const int64_t* offA,
   int64_t* doa = static_cast<int64_t*>(c->bOa.ptr);
   SS_CUDA(cudaMemcpyAsync(dn, n, sizeof(int) * size_t(nsys), cudaMemcpyHostToDevice, c->stream));
   SS_CUDA(cudaMemcpyAsync(doa, offA, sizeof(int64_t) * size_t(nsys), cudaMemcpyHostToDevice, c->stream));
-  const int grid = (nq + 255) / 256;
+  const int per = draws_per_warp(nq, c->num_sms);
+  const int64_t per_block = int64_t(kDrawThreads / 32) * per;
+  const int grid = int((nq + per_block - 1) / per_block);
   if (is_device_ptr(C)) {
-    matom_sample_kernel<<<grid, 256, 0, c->stream>>>(nq, nsys, dn, doa, C, sys, level, z, target);
+    matom_sample_kernel<<<grid, kDrawThreads, 0, c->stream>>>(nq, per, nsys, dn, doa, C, sys, level, z, target);
     SS_CUDA(cudaGetLastError());
     SS_CUDA(cudaStreamSynchronize(c->stream));
     return 0;
@@ -1109,7 +1111,7 @@ static int run_matom_sample(int nq, int nsys, const int* n, const int64_t* offA,
   SS_CUDA(cudaMemcpyAsync(ds, sys, sizeof(int) * size_t(nq), cudaMemcpyHostToDevice, c->stream));
   SS_CUDA(cudaMemcpyAsync(dl, level, sizeof(int) * size_t(nq), cudaMemcpyHostToDevice, c->stream));
   SS_CUDA(cudaMemcpyAsync(dz, z, sizeof(double) * size_t(nq), cudaMemcpyHostToDevice, c->stream));
-  matom_sample_kernel<<<grid, 256, 0, c->stream>>>(nq, nsys, dn, doa, dC, ds, dl, dz, dt);
+  matom_sample_kernel<<<grid, kDrawThreads, 0, c->stream>>>(nq, per, nsys, dn, doa, dC, ds, dl, dz, dt);
   SS_CUDA(cudaGetLastError());
   SS_CUDA(cudaMemcpyAsync(target, dt, sizeof(int) * size_t(nq), cudaMemcpyDeviceToHost, c->stream));
   SS_CUDA(cudaStreamSynchronize(c->stream));
