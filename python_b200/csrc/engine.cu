@@ -83,6 +83,7 @@ static const int kSmallNP[] = {
 #undef SS_SMALL_CLASS
 };
 constexpr int kSmallClasses = int(sizeof(kSmallNP) / sizeof(kSmallNP[0]));
+constexpr int kMaxSmallN = 32;   // the largest order of the family: one row per lane of a warp
 // padded orders of the CTA classes (cta_classes.inc, chosen by python_b200/autotune.py)
 static const int kCtaP[] = {
 #define SS_CTA_CLASS(I, P, NT, RG, CC, PW, GM, MINB) P,
@@ -131,6 +132,7 @@ static KernelSpec small_spec(int cls, int mode) {
                ? reinterpret_cast<const void*>(&small_mixed_solve_kernel<NP, G>)        \
                : reinterpret_cast<const void*>(&small_exact_kernel<KIND, NP, G>);       \
     k.sys_per_block = kSmallThreads / G;                                                \
+    k.dyn_smem = small_smem_bytes<NP, G>();                                             \
     break;
   switch (cls) {
 #include "small_classes.inc"
@@ -376,7 +378,8 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
   // Certified inverses (SIROCCO_FAST) go to the Gauss-Jordan classes; each also
   // has a place in the fallback list of its exact class (small or CTA family).
   const bool cert = (kind == kInvert && mode == SIROCCO_FAST);
-  std::vector<int> small_l[kSmallClasses], cta_l[kCtaClasses], glob_l, cgj_l[kCgjClasses], cgjl_l;
+  std::vector<int> small_n[kMaxSmallN + 1], small_l[kSmallClasses], cta_l[kCtaClasses], glob_l, cgj_l[kCgjClasses],
+      cgjl_l;
   int small_fb[kSmallClasses] = {}, cta_fb[kCtaClasses] = {};
   for (int s = 0; s < nsys; ++s) {
     const int ns = n[s];
@@ -399,9 +402,14 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
       cta_fb[cta_class(ns)]++;
       continue;
     }
-    if ((c = small_class(ns)) >= 0) small_l[c].push_back(s);
+    if (ns <= kMaxSmallN) small_n[ns].push_back(s);
     else if ((c = cta_class(ns)) >= 0) cta_l[c].push_back(s);
     else glob_l.push_back(s);
+  }
+  // systems of one order one after another: the groups of a warp take the same steps
+  for (int ns = 1; ns <= kMaxSmallN; ++ns) {
+    std::vector<int>& l = small_l[small_class(ns)];
+    l.insert(l.end(), small_n[ns].begin(), small_n[ns].end());
   }
   // fallback lists: one per exact class that certified systems belong to
   int small_fbi[kSmallClasses], cta_fbi[kCtaClasses];

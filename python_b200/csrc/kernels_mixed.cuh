@@ -42,9 +42,9 @@ template <int NP, int G>
 __global__ void __launch_bounds__(kSmallThreads)
 small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
   constexpr int GPB = kSmallThreads / G;
-  constexpr int S = SmallSmem<NP>::S;
   constexpr double kFloor = 1.0e-22;          // significance floor of a component (x_j / sum |x|)
-  __shared__ __align__(16) SmallSmem<NP> smem_all[GPB];
+  extern __shared__ __align__(16) unsigned char small_dsm[];
+  SmallSmem<NP>* smem_all = reinterpret_cast<SmallSmem<NP>*>(small_dsm);   // [GPB]
 
   const int grp = threadIdx.x / G;
   const int lane = threadIdx.x % G;
@@ -60,6 +60,7 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
     double* __restrict__ xg = bv.out + ov;
     small_stage<NP, G>(sm, bv.A + bv.offA[s], n, lane, gmask);
     const bool act = lane < n;
+    const int S = small_stride(n);
 
     // ---- 1. equilibration -------------------------------------------------
     double rmax = 0.0;
@@ -202,7 +203,7 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
         if (act) sm.xs[lane] = xj;
         __syncwarp(gmask);
         double worst;
-        const int code = small_residual_code<NP, G>(sm, bv.A + bv.offA[s], bg, n, lane, gmask, &worst);
+        const int code = small_residual_code<NP, G>(sm, act ? bg[lane] : 0.0, n, lane, gmask, &worst);
         // how close could the reference's own residual test come to 1e-6?
         double risk = 0.0;
         if (act) {
@@ -225,7 +226,7 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
 
     int code;
     if (fallback) {
-      code = small_exact_solve<NP, G>(sm, bv.A + bv.offA[s], bg, xg, n, lane, gmask);
+      code = small_exact_solve<NP, G>(sm, act ? bg[lane] : 0.0, xg, n, lane, gmask);
       diagbits |= kDiagFallback;
     } else {
       for (int k = lane; k < n; k += G) xg[k] = sm.xs[k];

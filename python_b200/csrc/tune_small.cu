@@ -15,9 +15,11 @@ namespace {
 struct Candidate {
   int NP, G;
   const void* fn;
+  size_t smem;
 };
 
-#define SS_TUNE_SMALL(NP, G) {NP, G, reinterpret_cast<const void*>(&ss::small_exact_kernel<ss::kSolve, NP, G>)},
+#define SS_TUNE_SMALL(NP, G) \
+  {NP, G, reinterpret_cast<const void*>(&ss::small_exact_kernel<ss::kSolve, NP, G>), ss::small_smem_bytes<NP, G>()},
 const Candidate kCand[] = {
 #include "tune_small_candidates.inc"
 };
@@ -48,7 +50,8 @@ int sirocco_tune_time(int i, int nsys, const int* d_n, const int64_t* d_offA, co
   const Candidate& c = kCand[i];
   cudaError_t e;
   int nb = 0, dev = 0, sms = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, c.fn, ss::kSmallThreads, 0))) return int(e);
+  if ((e = cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(c.smem)))) return int(e);
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, c.fn, ss::kSmallThreads, c.smem))) return int(e);
   if (nb < 1) return -2;
   if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return int(e);
   const int per_block = ss::kSmallThreads / c.G;
@@ -72,7 +75,7 @@ int sirocco_tune_time(int i, int nsys, const int* d_n, const int64_t* d_offA, co
   int rc = 0;
   for (int r = 0; r <= reps && rc == 0; ++r) {   // launch 0 warms up
     cudaEventRecord(e0);
-    if ((e = cudaLaunchKernel(c.fn, dim3(grid), dim3(ss::kSmallThreads), args, 0, 0))) rc = int(e);
+    if ((e = cudaLaunchKernel(c.fn, dim3(grid), dim3(ss::kSmallThreads), args, c.smem, 0))) rc = int(e);
     cudaEventRecord(e1);
     if (!rc && (e = cudaEventSynchronize(e1))) rc = int(e);
     float t = 0.f;
