@@ -33,6 +33,7 @@
 #include "kernels_cta.cuh"
 #include "kernels_global.cuh"
 #include "kernels_ionasm.cuh"
+#include "kernels_ionlock.cuh"
 #include "kernels_matom.cuh"
 #include "kernels_matomasm.cuh"
 #include "kernels_mixed.cuh"
@@ -1134,8 +1135,8 @@ static int run_matom_sample(int nq, int nsys, const int* n, const int64_t* offA,
 // each element's block is the conservation row), so LU with partial pivoting on
 // the full matrix only ever meets exact zeros outside a block: the per-element
 // solves give the full matrix's solution and codes bit for bit.
-constexpr double kDensityMin = 1.0e-20;   // atomic.h:9
-constexpr double kFracError = 0.03;       // python.h:1212
+constexpr double kDensityMin = kLockDensityMin;
+constexpr double kFracError = kLockFracError;
 constexpr int kMaxIterations = 200;       // python.h:1211
 
 // Elements own consecutive ion ranges that together cover every ion once.
@@ -1490,6 +1491,94 @@ static int run_ion_rate_matrices(const sirocco_ion_table* t, int ncell, const si
   return 0;
 }
 
+// Deals the elements to the warps of a cell, the largest first to the least
+// loaded: as many warps as the largest element's chain leaves room for.
+static int ion_lock_warps(int nelem, const int* elem_n, std::vector<int>& start, std::vector<int>& elems) {
+  std::vector<int> order(nelem);
+  for (int e = 0; e < nelem; ++e) order[e] = e;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return elem_n[x] > elem_n[y]; });
+  auto cost = [&](int e) { return int64_t(elem_n[e]) + 4; };   // steps of about equal length, and the fixed part
+  int64_t total = 0;
+  for (int e = 0; e < nelem; ++e) total += cost(e);
+  const int64_t top = cost(order[0]);
+  const int nw = int(std::min<int64_t>(kIonLockWarps, std::max<int64_t>(1, (total + top / 2) / top)));
+  std::vector<std::vector<int>> of(nw);
+  std::vector<int64_t> load(nw, 0);
+  for (int e : order) {
+    const int w = int(std::min_element(load.begin(), load.end()) - load.begin());
+    of[w].push_back(e);
+    load[w] += cost(e);
+  }
+  start.assign(1, 0);
+  elems.clear();
+  for (auto& l : of) {
+    elems.insert(elems.end(), l.begin(), l.end());
+    start.push_back(int(elems.size()));
+  }
+  return nw;
+}
+
+// The n_e iteration with every round on the GPU (kernels_ionlock.cuh): exact
+// solves of elements of at most kMaxSmallN ions.
+template <int NPM>
+static int launch_ion_lock(Context* c, const IonAsmView& v, const IonLockView& lv, int warps) {
+  const size_t smem = ion_lock_smem<NPM>(warps, v.nions);
+  const auto fn = &ion_lockstep_kernel<NPM>;
+  SS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  int nb = 0;
+  SS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * warps, smem));
+  fn<<<std::min(lv.ncell, std::max(1, nb) * c->num_sms), 32 * warps, smem, c->stream>>>(v, lv);
+  SS_CUDA(cudaGetLastError());
+  return 0;
+}
+
+static int run_ion_lockstep_device(Context* c, IonAsmView& v, const sirocco_ion_table* t, int ncell, int h_elem,
+                                   const double* elem_dens, const std::vector<int>& elem_of, double* ne, double* den,
+                                   int* status, int* iters) {
+  const size_t nc = size_t(ncell), nions = size_t(t->nions), nelem = size_t(t->nelem);
+  std::vector<int> start, elems;
+  const int warps = ion_lock_warps(t->nelem, t->elem_n, start, elems);
+  std::vector<int> ints(1, 0);   // the queue
+  ints.insert(ints.end(), elem_of.begin(), elem_of.end());
+  ints.insert(ints.end(), start.begin(), start.end());
+  ints.insert(ints.end(), elems.begin(), elems.end());
+  int rc;
+  if ((rc = c->bIL.ensure(sizeof(int) * ints.size())) || (rc = c->bIS.ensure(sizeof(double) * nc * nelem)) ||
+      (rc = c->bIX.ensure(sizeof(double) * nc * (nions + 1))) || (rc = c->bISt.ensure(sizeof(int) * 2 * nc)))
+    return rc;
+  int* di = static_cast<int*>(c->bIL.ptr);
+  int* ds = static_cast<int*>(c->bISt.ptr);
+  double* dx = static_cast<double*>(c->bIX.ptr);
+  IonLockView lv;
+  lv.ncell = ncell;
+  lv.h_elem = h_elem;
+  lv.max_rounds = kMaxIterations;
+  lv.queue = di;
+  lv.elem_of = di + 1;
+  lv.warp_start = lv.elem_of + nions;
+  lv.warp_elem = lv.warp_start + start.size();
+  lv.dens = static_cast<const double*>(c->bIS.ptr);
+  lv.ne = dx;
+  lv.den = dx + nc;
+  lv.status = ds;
+  lv.iters = ds + nc;
+  SS_CUDA(cudaMemcpyAsync(di, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice, c->stream));
+  SS_CUDA(cudaMemcpyAsync(c->bIS.ptr, elem_dens, sizeof(double) * nc * nelem, cudaMemcpyHostToDevice, c->stream));
+  SS_CUDA(cudaMemcpyAsync(lv.ne, ne, sizeof(double) * nc, cudaMemcpyHostToDevice, c->stream));
+  SS_CUDA(cudaMemcpyAsync(lv.den, den, sizeof(double) * nc * nions, cudaMemcpyHostToDevice, c->stream));
+  const int top = *std::max_element(t->elem_n, t->elem_n + t->nelem);
+  if (top <= 16) rc = launch_ion_lock<16>(c, v, lv, warps);
+  else if (top <= 28) rc = launch_ion_lock<28>(c, v, lv, warps);
+  else rc = launch_ion_lock<32>(c, v, lv, warps);
+  if (rc) return rc;
+  SS_CUDA(cudaMemcpyAsync(ne, lv.ne, sizeof(double) * nc, cudaMemcpyDeviceToHost, c->stream));
+  SS_CUDA(cudaMemcpyAsync(den, lv.den, sizeof(double) * nc * nions, cudaMemcpyDeviceToHost, c->stream));
+  SS_CUDA(cudaMemcpyAsync(status, lv.status, sizeof(int) * nc, cudaMemcpyDeviceToHost, c->stream));
+  SS_CUDA(cudaMemcpyAsync(iters, lv.iters, sizeof(int) * nc, cudaMemcpyDeviceToHost, c->stream));
+  SS_CUDA(cudaStreamSynchronize(c->stream));
+  return 0;
+}
+
 static int run_ion_lockstep_rates(const sirocco_ion_table* t, int ncell, const sirocco_ion_rates* r, int h_elem,
                                   const double* elem_dens, double* ne, double* den, int* status, int* iters) {
   if (ncell == 0) return 0;
@@ -1504,6 +1593,11 @@ static int run_ion_lockstep_rates(const sirocco_ion_table* t, int ncell, const s
   int64_t blkA = 0;
   if ((rc = ion_asm_prepare(t, ncell, r, c, v, elem_of, blkA))) return rc;
   const int nions = t->nions, nelem = t->nelem;
+  // exact solves of elements that fit a warp run every round on the GPU; mixed
+  // mode and larger elements go round by round through the batched solve
+  if (c->mode != SIROCCO_MIXED && nions <= kIonLockMaxIons &&
+      *std::max_element(t->elem_n, t->elem_n + nelem) <= kMaxSmallN)
+    return run_ion_lockstep_device(c, v, t, ncell, h_elem, elem_dens, elem_of, ne, den, status, iters);
   std::vector<int> n, pc;
   std::vector<int64_t> offA, offv;
   std::vector<double> pne, ph1, ph2;

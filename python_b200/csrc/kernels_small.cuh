@@ -26,7 +26,7 @@ constexpr int kSmallThreads = 128;
 template <int NP>
 struct __align__(16) SmallSmem {
   static constexpr int S = NP + 1;   // odd row stride (in doubles) avoids bank conflicts
-  double stage[NP * S];              // A as loaded (solve: kept for the residual check)
+  double stage[NP * S];              // A as loaded (solve: kept for the residual check); comes first
   double u[NP * (NP + 3 - NP / 2)];  // the pivot rows by step (solve: small_urow; invert: the current one)
   double xs[NP];                     // solution in natural order
   float fpiv[NP];                    // broadcast pivot row (mixed path)
