@@ -1492,16 +1492,15 @@ static int run_ion_rate_matrices(const sirocco_ion_table* t, int ncell, const si
 }
 
 // Deals the elements to the warps of a cell, the largest first to the least
-// loaded: as many warps as the largest element's chain leaves room for.
+// loaded, on as many warps as there are elements, up to kIonLockWarps: a cell
+// that takes many rounds (200 where it never converges) is alone on the GPU at
+// the end, so a round's length counts for more than the warps that idle in it.
 static int ion_lock_warps(int nelem, const int* elem_n, std::vector<int>& start, std::vector<int>& elems) {
   std::vector<int> order(nelem);
   for (int e = 0; e < nelem; ++e) order[e] = e;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return elem_n[x] > elem_n[y]; });
   auto cost = [&](int e) { return int64_t(elem_n[e]) + 4; };   // steps of about equal length, and the fixed part
-  int64_t total = 0;
-  for (int e = 0; e < nelem; ++e) total += cost(e);
-  const int64_t top = cost(order[0]);
-  const int nw = int(std::min<int64_t>(kIonLockWarps, std::max<int64_t>(1, (total + top / 2) / top)));
+  const int nw = std::min(kIonLockWarps, nelem);
   std::vector<std::vector<int>> of(nw);
   std::vector<int64_t> load(nw, 0);
   for (int e : order) {

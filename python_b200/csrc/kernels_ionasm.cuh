@@ -50,55 +50,60 @@ constexpr int kIonAsmThreads = 128;
 __device__ __forceinline__ void ion_column(const IonAsmView& v, int cell, int f, int n, int cl, double xne, double nh1,
                                            double nh2, double* __restrict__ blk, int stride) {
   const int64_t rc = int64_t(cell) * v.nions;
-  for (int r = 0; r < n; ++r) blk[int64_t(r) * stride + cl] = (r == 0) ? 1.0 : 0.0;
   const int nn = f + cl;
-  const int flags = v.ion_flags[nn];
+  // every coefficient of the ion on its way before the first is used
+  const double pi = v.pi[rc + nn], rr = v.rr[rc + nn], di = v.di[rc + nn], qr = v.qr[rc + nn], dr = v.dr[rc + nn],
+               cxr = v.cxr[rc + nn];
+  const int flags = v.ion_flags[nn], lower = cl != 0 ? v.ion_flags[nn - 1] : 0, z = v.ion_z[nn],
+            istate = v.ion_istate[nn];
+  const int cx0 = v.cx_start[nn], cx1 = v.cx_start[nn + 1], in0 = v.in_start[nn], in1 = v.in_start[nn + 1];
+  for (int r = 0; r < n; ++r) blk[int64_t(r) * stride + cl] = (r == 0) ? 1.0 : 0.0;
   const bool top = flags & 1, has_di = flags & 2, has_dr = flags & 4;
   const bool below = cl + 1 < n;   // ion nn + 1 is of the same element
   double diag = 0.0, sub = 0.0, sup = 0.0;
   double inn[9];
 #pragma unroll
   for (int d = 0; d < 9; ++d) inn[d] = 0.0;
-      // photoionisation (:477-497)
-      if (!top) diag = sub_rn(diag, v.pi[rc + nn]);
-      if (!top && below) sub = add_rn(sub, v.pi[rc + nn]);
-      // direct ionisation (:501-520)
-      if (!top && has_di) diag = sub_rn(diag, mul_rn(xne, v.di[rc + nn]));
-      if (!top && below && has_di) sub = add_rn(sub, mul_rn(xne, v.di[rc + nn]));
-      // radiative and three-body recombination (:525-544)
-      if (cl != 0) {
-        const double t = mul_rn(xne, add_rn(v.rr[rc + nn], mul_rn(xne, v.qr[rc + nn])));
-        diag = sub_rn(diag, t);
-        sup = add_rn(sup, t);
-      }
-      // dielectronic recombination (:548-572); the populating term takes the
-      // flag of the lower ion
-      if (cl != 0 && has_dr) diag = sub_rn(diag, mul_rn(xne, v.dr[rc + nn]));
-      if (cl != 0 && (v.ion_flags[nn - 1] & 4)) sup = add_rn(sup, mul_rn(xne, v.dr[rc + nn]));
-      // charge-exchange recombination (:576-586); the term above a neutral ion
-      // falls outside the block and is zero (checked on the host)
-      if (v.ncx > 0 && v.ion_z[nn] != 1 && v.ion_istate[nn] != 0) {
-        const double t = mul_rn(v.cxr[rc + nn], nh1);
-        diag = sub_rn(diag, t);
-        if (cl != 0) sup = add_rn(sup, t);
-      }
-      // charge-exchange ionisation against hydrogen (:590-596), entries in order
-      for (int k = v.cx_start[nn]; k < v.cx_start[nn + 1]; ++k) {
-        const double t = mul_rn(v.cxi[int64_t(cell) * v.ncx + v.cx_idx[k]], nh2);
-        diag = sub_rn(diag, t);
-        sub = add_rn(sub, t);
-      }
-      // inner-shell ionisation with electron yields (:599-613), rates in order
-      const int nel = min(v.ion_z[nn] - v.ion_istate[nn] + 1, 11);
-      for (int k = v.in_start[nn]; k < v.in_start[nn + 1]; ++k) {
-        const double rate = v.inner[int64_t(cell) * v.n_inner + v.in_idx[k]];
-        const double* __restrict__ prob = v.yield + int64_t(v.in_yield[k]) * 10;
-        diag = sub_rn(diag, rate);
-        if (nel > 1) sub = add_rn(sub, mul_rn(rate, prob[0]));
+  // photoionisation (:477-497)
+  if (!top) diag = sub_rn(diag, pi);
+  if (!top && below) sub = add_rn(sub, pi);
+  // direct ionisation (:501-520)
+  if (!top && has_di) diag = sub_rn(diag, mul_rn(xne, di));
+  if (!top && below && has_di) sub = add_rn(sub, mul_rn(xne, di));
+  // radiative and three-body recombination (:525-544)
+  if (cl != 0) {
+    const double t = mul_rn(xne, add_rn(rr, mul_rn(xne, qr)));
+    diag = sub_rn(diag, t);
+    sup = add_rn(sup, t);
+  }
+  // dielectronic recombination (:548-572); the populating term takes the
+  // flag of the lower ion
+  if (cl != 0 && has_dr) diag = sub_rn(diag, mul_rn(xne, dr));
+  if (cl != 0 && (lower & 4)) sup = add_rn(sup, mul_rn(xne, dr));
+  // charge-exchange recombination (:576-586); the term above a neutral ion
+  // falls outside the block and is zero (checked on the host)
+  if (v.ncx > 0 && z != 1 && istate != 0) {
+    const double t = mul_rn(cxr, nh1);
+    diag = sub_rn(diag, t);
+    if (cl != 0) sup = add_rn(sup, t);
+  }
+  // charge-exchange ionisation against hydrogen (:590-596), entries in order
+  for (int k = cx0; k < cx1; ++k) {
+    const double t = mul_rn(v.cxi[int64_t(cell) * v.ncx + v.cx_idx[k]], nh2);
+    diag = sub_rn(diag, t);
+    sub = add_rn(sub, t);
+  }
+  // inner-shell ionisation with electron yields (:599-613), rates in order
+  const int nel = min(z - istate + 1, 11);
+  for (int k = in0; k < in1; ++k) {
+    const double rate = v.inner[int64_t(cell) * v.n_inner + v.in_idx[k]];
+    const double* __restrict__ prob = v.yield + int64_t(v.in_yield[k]) * 10;
+    diag = sub_rn(diag, rate);
+    if (nel > 1) sub = add_rn(sub, mul_rn(rate, prob[0]));
   #pragma unroll
-        for (int d = 2; d <= 10; ++d)
-          if (d < nel) inn[d - 2] = add_rn(inn[d - 2], mul_rn(rate, prob[d - 1]));
-      }
+    for (int d = 2; d <= 10; ++d)
+      if (d < nel) inn[d - 2] = add_rn(inn[d - 2], mul_rn(rate, prob[d - 1]));
+  }
   // the structured entries over the zeros, in this lane's program order
   if (cl != 0) blk[int64_t(cl) * stride + cl] = diag;
   if (below) blk[int64_t(cl + 1) * stride + cl] = sub;

@@ -7,10 +7,8 @@
 // (small_exact_solve, a warp per system), then warp 0 floors the populations,
 // sums n_e in ion order and decides.  Nothing but the converged n_e and
 // populations leaves the SM, and the host takes part only before and after.
-// What bounds it is the chain of the largest element's solve, once per round;
-// the elements are dealt to as many warps as keep that chain the longest
-// (host, ion_lock_warps), so that a cell occupies no more of the SM than it
-// can use.  Rounds driven by the host (a layout, a plan, five launches and four
+// What bounds it is the chain of the largest element's solve, once per round,
+// times the rounds of the cell that takes the most.  Rounds driven by the host (a layout, a plan, five launches and four
 // copies each) took 20.0 ms for 4,096 cells of five elements; LOCK_NOW.
 #pragma once
 #include "kernels_ionasm.cuh"
@@ -43,23 +41,17 @@ size_t ion_lock_smem(int warps, int nions) {
   return sizeof(SmallSmem<NPM>) * size_t(warps) + sizeof(double) * 2 * size_t(nions);
 }
 
-// raw: a warp's scratch; the matrix is staged at its start, as in SmallSmem
-template <int NP>
-__device__ __forceinline__ int ion_lock_solve(unsigned char* raw, double* x, int n, int lane) {
-  return small_exact_solve<NP, 32>(*reinterpret_cast<SmallSmem<NP>*>(raw), lane == 0 ? 1.0 : 0.0, x, n, lane,
-                                   0xffffffffu);
-}
-
-// NPM: padded order that holds every element (<= 32)
+// NPM: padded order that holds every element (<= 32).  Every element goes
+// through the same unrolled steps, small ones through the first few of them:
+// with a size class each, the warps' code no longer fits the instruction cache
+// together and a pivot step at n = 27 takes 740 cycles instead of 430.
 template <int NPM>
 __global__ void __launch_bounds__(32 * kIonLockWarps, NPM > 28 ? 3 : 4) ion_lockstep_kernel(IonAsmView v, IonLockView lv) {
   extern __shared__ __align__(16) unsigned char lock_dsm[];
   __shared__ int s_cell, s_sing, s_state;    // s_state: 0 another round, 1 converged, 2 singular
   __shared__ double s_ne, s_h1, s_h2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  unsigned char* raw = lock_dsm + sizeof(SmallSmem<NPM>) * size_t(warp);
-  static_assert(sizeof(SmallSmem<8>) <= sizeof(SmallSmem<NPM>) && sizeof(SmallSmem<16>) <= sizeof(SmallSmem<NPM>),
-                "scratch of the largest order");
+  SmallSmem<NPM>& sm = reinterpret_cast<SmallSmem<NPM>*>(lock_dsm)[warp];
   double* nd = reinterpret_cast<double*>(lock_dsm + sizeof(SmallSmem<NPM>) * size_t(nw));   // [nions]
   double* term = nd + v.nions;                                                              // [nions]
 
@@ -96,13 +88,11 @@ __global__ void __launch_bounds__(32 * kIonLockWarps, NPM > 28 ? 3 : 4) ion_lock
       const double xne = s_ne, nh1 = s_h1, nh2 = s_h2;
       for (int q = lv.warp_start[warp]; q < lv.warp_start[warp + 1]; ++q) {
         const int e = lv.warp_elem[q], n = v.elem_n[e], f = v.elem_first[e];
-        if (lane < n) ion_column(v, cell, f, n, lane, xne, nh1, nh2, reinterpret_cast<double*>(raw),
-                                 small_stride(n));
+        if (lane < n) ion_column(v, cell, f, n, lane, xne, nh1, nh2, sm.stage, small_stride(n));
         __syncwarp();
-        int code;
-        if (n <= 8) code = ion_lock_solve<8>(raw, nd + f, n, lane);
-        else if (n <= 16) code = ion_lock_solve<16>(raw, nd + f, n, lane);
-        else code = ion_lock_solve<NPM>(raw, nd + f, n, lane);
+        // the iteration looks at nothing but code 4: no residual check
+        const int code =
+            small_exact_solve<NPM, 32, false>(sm, lane == 0 ? 1.0 : 0.0, nd + f, n, lane, 0xffffffffu);
         if (code == kSolveSingular && lane == 0) s_sing = 1;
         __syncwarp();
       }

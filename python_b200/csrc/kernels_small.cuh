@@ -319,7 +319,9 @@ __device__ __noinline__ double small_upper_general(SmallSmem<NP>& sm, int n, int
 // lane used to walk it, a load, a product and a difference per entry).
 // 4,096 systems of order 27: 66 -> 43 us; 200,000 of the orders one cell carries
 // (2-27): 770 -> 522 us.
-template <int NP, int G>
+// CHECK: false leaves the residual check out (code 0 or 4), for callers to whom
+// codes 2 and 3 mean nothing.
+template <int NP, int G, bool CHECK = true>
 __device__ __forceinline__ int small_exact_solve(SmallSmem<NP>& sm, double bi, double* __restrict__ xg, int n,
                                                  int lane, unsigned mask) {
   static_assert(NP % 4 == 0, "pivot rows move in pairs");
@@ -425,10 +427,13 @@ __device__ __forceinline__ int small_exact_solve(SmallSmem<NP>& sm, double bi, d
     }
   }
   if (__any_sync(mask, far >= kDivFar && !sing)) xv = small_upper_general<NP, G>(sm, n, lane, mask);
-  if (lane < n) sm.xs[lane] = xv;
-  __syncwarp(mask);
-  double worst;
-  const int code = small_residual_code<NP, G>(sm, bi, n, lane, mask, &worst);
+  int code = kOk;
+  if (CHECK) {
+    if (lane < n) sm.xs[lane] = xv;
+    __syncwarp(mask);
+    double worst;
+    code = small_residual_code<NP, G>(sm, bi, n, lane, mask, &worst);
+  }
   if (lane < n && !sing) xg[lane] = xv;
   return sing ? kSolveSingular : code;
 }
