@@ -259,6 +259,7 @@ struct Bucket {
   int phase;      // 1: certified kernels and directly listed systems; 2: fallback lists
   int fb;         // phase 2: index of the fallback list this launch serves
   int q;          // streamed certified inverses: index of the launch's queue counter
+  bool fills;     // small systems that fill the GPU at least twice over
 };
 
 }  // namespace ss
@@ -468,6 +469,7 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
     if (rc) return rc;
     const int blocks_needed = (b.count + b.spec.sys_per_block - 1) / b.spec.sys_per_block;
     b.grid = std::max(1, std::min(blocks_needed * b.spec.cluster, b.spec.max_ctas));
+    b.fills = fam == kFamSmall && fb < 0 && blocks_needed >= 2 * b.spec.max_ctas;
     if (fam == kFamGlobal && kind == kSolve) {
       b.slab = (int64_t(cls) * cls + 31) / 32 * 32;
       b.scratch_off = scratch_elems;
@@ -526,10 +528,16 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
   p->scratch_elems = scratch_elems;
   p->own_scratch = alloc_scratch;
   if (alloc_scratch && scratch_elems > 0) SS_CUDA(cudaMalloc(&p->d_scratch, sizeof(double) * scratch_elems));
-  // one side stream per bucket of a phase beyond the first
-  size_t per_phase[3] = {0, 0, 0};
-  for (auto& b : p->buckets) per_phase[b.phase]++;
-  for (size_t i = 1; i < std::max(per_phase[1], per_phase[2]); ++i) {
+  // one side stream per forked bucket of a phase (run_phase)
+  size_t forked[3] = {0, 0, 0};
+  bool queued[3] = {false, false, false};
+  for (auto& b : p->buckets) {
+    if (b.fills) queued[b.phase] = true;
+    else forked[b.phase]++;
+  }
+  for (int ph : {1, 2})
+    if (!queued[ph] && forked[ph] > 0) forked[ph]--;   // the first one runs on the caller's stream
+  for (size_t i = 0; i < std::max(forked[1], forked[2]); ++i) {
     cudaStream_t st;
     SS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     p->side.push_back(st);
@@ -603,24 +611,31 @@ static int launch_bucket(const sirocco_plan* p, const Bucket& b, const double* A
   return 0;
 }
 
-// The buckets of one phase, forked onto the side streams and joined back into st.
+// The buckets of one phase, forked onto the side streams and joined back into
+// st.  Small-system buckets that fill the GPU on their own run one after another
+// instead: their kernels are unrolled over the order, and two of them on one SM
+// evict each other's code from the instruction cache (200,000 systems of orders
+// 2-27: 522 us forked, 506 us in turn).
 static int run_phase(sirocco_plan* p, int phase, const double* A, const double* bvec, double* out, int* status,
                      int* diag, cudaStream_t st) {
-  std::vector<const Bucket*> bs;
+  std::vector<const Bucket*> bs, queue;   // queue: one after another on st
   for (auto& b : p->buckets)
-    if (b.phase == phase) bs.push_back(&b);
-  if (bs.empty()) return 0;
-  if (bs.size() == 1) return launch_bucket(p, *bs[0], A, bvec, out, status, diag, st);
-  SS_CUDA(cudaEventRecord(p->ev_fork, st));
-  for (size_t i = 1; i < bs.size(); ++i) SS_CUDA(cudaStreamWaitEvent(p->side[i - 1], p->ev_fork, 0));
-  int rc = launch_bucket(p, *bs[0], A, bvec, out, status, diag, st);
-  if (rc) return rc;
-  for (size_t i = 1; i < bs.size(); ++i) {
-    rc = launch_bucket(p, *bs[i], A, bvec, out, status, diag, p->side[i - 1]);
-    if (rc) return rc;
-    SS_CUDA(cudaEventRecord(p->ev[i - 1], p->side[i - 1]));
+    if (b.phase == phase) (b.fills ? queue : bs).push_back(&b);
+  if (!bs.empty()) {
+    if (queue.empty()) {
+      queue.push_back(bs.front());
+      bs.erase(bs.begin());
+    }
+    if (!bs.empty()) SS_CUDA(cudaEventRecord(p->ev_fork, st));
   }
-  for (size_t i = 1; i < bs.size(); ++i) SS_CUDA(cudaStreamWaitEvent(st, p->ev[i - 1], 0));
+  for (size_t i = 0; i < bs.size(); ++i) SS_CUDA(cudaStreamWaitEvent(p->side[i], p->ev_fork, 0));
+  for (const Bucket* b : queue)
+    if (int rc = launch_bucket(p, *b, A, bvec, out, status, diag, st)) return rc;
+  for (size_t i = 0; i < bs.size(); ++i) {
+    if (int rc = launch_bucket(p, *bs[i], A, bvec, out, status, diag, p->side[i])) return rc;
+    SS_CUDA(cudaEventRecord(p->ev[i], p->side[i]));
+  }
+  for (size_t i = 0; i < bs.size(); ++i) SS_CUDA(cudaStreamWaitEvent(st, p->ev[i], 0));
   return 0;
 }
 

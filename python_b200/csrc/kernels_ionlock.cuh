@@ -8,8 +8,10 @@
 // sums n_e in ion order and decides.  Nothing but the converged n_e and
 // populations leaves the SM, and the host takes part only before and after.
 // What bounds it is the chain of the largest element's solve, once per round,
-// times the rounds of the cell that takes the most.  Rounds driven by the host (a layout, a plan, five launches and four
-// copies each) took 20.0 ms for 4,096 cells of five elements; LOCK_NOW.
+// times the rounds of the cell that takes the most.  4,096 cells of five elements
+// took 21.1 ms a call with rounds driven by the host (a layout, a plan, five
+// launches and four copies each); now 4.9 ms, of which 3 are the 200 rounds of a
+// cell that never converges (15 us each) and about 1.5 the copies in and out.
 #pragma once
 #include "kernels_ionasm.cuh"
 #include "kernels_small.cuh"
