@@ -67,6 +67,7 @@ enum Family : int { kFamSmall = 0, kFamCta = 1, kFamGlobal = 2, kFamCgj = 3, kFa
 
 struct KernelSpec {
   const void* fn = nullptr;
+  const void* fn_epi = nullptr;   // certified family: the kernel with the macro-atom epilogue
   int threads = 0;
   size_t dyn_smem = 0;
   int sys_per_block = 1;
@@ -172,6 +173,7 @@ static KernelSpec cgj_spec(int cls) {
   case I: {                                                                              \
     using Sh = CgjShape<P, WGR, WGC, CL, MINB, ST>;                                      \
     k.fn = reinterpret_cast<const void*>(&cgj_inverse_kernel<P, WGR, WGC, CL, MINB, ST>); \
+    k.fn_epi = reinterpret_cast<const void*>(&cgj_inverse_kernel<P, WGR, WGC, CL, MINB, ST, true>); \
     k.threads = Sh::NTH;                                                             \
     k.dyn_smem = Sh::dyn_smem;                                                       \
     k.cluster = CL;                                                                  \
@@ -209,8 +211,9 @@ static int finish_spec(KernelSpec& k) {
     set_error("no kernel for this size class");
     return SIROCCO_ESIZE;
   }
-  if (k.dyn_smem > 0)
-    SS_CUDA(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.dyn_smem)));
+  for (const void* f : {k.fn, k.fn_epi})
+    if (f && k.dyn_smem > 0)
+      SS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.dyn_smem)));
   int nb = 0;
   SS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn, k.threads, k.dyn_smem));
   if (nb < 1) {
@@ -589,7 +592,7 @@ static int launch_bucket(const sirocco_plan* p, const Bucket& b, const double* A
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = b.spec.cluster > 1 ? 1 : 0;
-    SS_CUDA(cudaLaunchKernelExC(&cfg, b.spec.fn, args));
+    SS_CUDA(cudaLaunchKernelExC(&cfg, (ep.R || ep.C) ? b.spec.fn_epi : b.spec.fn, args));
   } else if (b.fam == kFamGlobal) {
     int nmax = b.cls;
     double* scratch = p->d_scratch ? p->d_scratch + b.scratch_off : nullptr;

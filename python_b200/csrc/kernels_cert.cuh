@@ -159,8 +159,8 @@ struct CgjShape {
   static_assert(buf % 2 == 0 && off_dg % 2 == 0, "16-byte aligned buffers");
   static_assert(!STAGE || LB <= 32, "one lane of the pivot warp issues each block's copy");
   static_assert(dyn_smem <= 232448, "one CTA's shared memory");
-  static_assert(((LP + 31) / 32) * 32 * 33 <= off_dg && (LP + 31) / 32 <= NW,
-                "the running-total tiles fit the panel buffers, one tile warp per 32 rows");
+  static_assert(3 * LP * 16 <= off_dg && (LP + 31) / 32 <= NW,
+                "three running-total pieces fit the panel buffers, one tile warp per 32 rows");
 };
 
 __device__ __forceinline__ unsigned cluster_rank() {
@@ -174,6 +174,21 @@ __device__ __forceinline__ unsigned cluster_rank() {
 template <int CL>
 __device__ __forceinline__ void cluster_barrier() {
   if (CL > 1) cooperative_groups::this_cluster().sync();
+  else __syncthreads();
+}
+
+// Its two halves: writes made before the arrival are visible after the wait.
+template <int CL>
+__device__ __forceinline__ void cluster_arrive() {
+  if (CL > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+}
+template <int CL>
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  if (CL > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+}
+template <int CL>
+__device__ __forceinline__ void cluster_wait() {
+  if (CL > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   else __syncthreads();
 }
 
@@ -347,7 +362,9 @@ __device__ __forceinline__ void warp_inv8_refined(double& d0, double& d1, int la
   }
 }
 
-template <int P, int WGR, int WGC, int CL, int MINB, bool STAGE = true>
+// EPI: the macro-atom epilogue is compiled in (CertEpi); without it the kernel
+// writes the inverse and its registers are the factorisation's alone.
+template <int P, int WGR, int WGC, int CL, int MINB, bool STAGE = true, bool EPI = false>
 __global__ void __launch_bounds__(32 * WGR * WGC + 32, MINB)
 cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
   using S = CgjShape<P, WGR, WGC, CL, MINB, STAGE>;
@@ -366,10 +383,18 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
   const int cnt = batch_count(bv);
 
   // local row (in this CTA) and global row of this lane's row in sub-block row i,
-  // global column of its column e in sub-block column j
+  // global column of its column e in sub-block column j, in the order the
+  // factorisation counts them
   auto lrow = [&](int i) -> int { return (wr + WGR * i) * 8 + g; };
   auto grow = [&](int i) -> int { return ((wr + WGR * i) * CL + rank) * 8 + g; };
   auto gcol = [&](int j, int e) -> int { return (wc + WGC * j) * 8 + 2 * t + e; };
+  // ... and in the matrix: inside every block of 8, its row and column q sit at
+  // q / 2 + 4 (q % 2).  The same order for both, so nothing changes but the
+  // order of the pivots; the four lanes of a fragment row then read and write
+  // 32 contiguous bytes (2t, 2t + 1 per lane touched half of two sectors)
+  const int pg = (g >> 1) + 4 * (g & 1);
+  auto mrow = [&](int i) -> int { return ((wr + WGR * i) * CL + rank) * 8 + pg; };
+  auto mcol = [&](int j, int e) -> int { return (wc + WGC * j) * 8 + t + 4 * e; };
   auto bufp = [&](int kblk) -> double* { return sm + (kblk & 1) * S::buf; };
   double W[WR][WC][2];
   // block steps of the current matrix: those whose pivot block holds no row
@@ -563,18 +588,18 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
       if (STAGE) {
         uintptr_t b0, b1;
         const int shift = block_span(s, 0, b0, b1) ? int((b0 >> 3) & 1) : 0;
-        const double* slot = stage + shift + g * n;
+        const double* slot = stage + shift + pg * n;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int c = 2 * t + e;
-          d[e] = (g < n && c < n) ? slot[c] : ((g == c) ? 1.0 : 0.0);
+          const int c = t + 4 * e;
+          d[e] = (pg < n && c < n) ? slot[c] : ((pg == c) ? 1.0 : 0.0);
         }
       } else {
         const double* Ag = bv.A + bv.offA[s];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int c = 2 * t + e;
-          d[e] = (g < n && c < n) ? __ldg(Ag + int64_t(g) * n + c) : ((g == c) ? 1.0 : 0.0);
+          const int c = t + 4 * e;
+          d[e] = (pg < n && c < n) ? __ldg(Ag + int64_t(pg) * n + c) : ((pg == c) ? 1.0 : 0.0);
         }
       }
       pivot_inverse(0, d[0], d[1]);
@@ -588,12 +613,12 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
       const double* __restrict__ Ag = bv.A + bv.offA[s];
 #pragma unroll
       for (int i = 0; i < WR; ++i) {
-        const int r = grow(i);
+        const int r = mrow(i);
 #pragma unroll
         for (int j = 0; j < WC; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const int c = gcol(j, e);
+            const int c = mcol(j, e);
             W[i][j][e] = __ldg(Ag + ((r < n && c < n) ? int64_t(r) * n + c : 0));
           }
       }
@@ -604,14 +629,14 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
         uintptr_t b0, b1;
         const int lb = wr + WGR * i;
         const int shift = (STAGE && block_span(s, lb, b0, b1)) ? int((b0 >> 3) & 1) : 0;
-        const double* slot = stage + lb * S::SLOT + shift + g * n;
-        const int r = grow(i);
+        const double* slot = stage + lb * S::SLOT + shift + pg * n;
+        const int r = mrow(i);
         double part = 0.0;
 #pragma unroll
         for (int j = 0; j < WC; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const int c = gcol(j, e);
+            const int c = mcol(j, e);
             const double a = (r < n && c < n) ? (STAGE ? slot[c] : W[i][j][e]) : ((r == c) ? 1.0 : 0.0);
             W[i][j][e] = a;
             if (c == r) {
@@ -816,70 +841,117 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
       }
     }
 
-    // ---- store N^-1, or B = N^-1 diag(R) with the fused epilogue
+    // ---- store N^-1, or B = N^-1 diag(R) with the fused epilogue.  The cluster's
+    // CTAs announce that they are done with the panel buffers before the stores
+    // and wait for one another after them: a release behind the stores would
+    // hold every warp until they have all landed.
+    cluster_arrive<CL>();
+    if (EPI && ep.R && tile) {
+      const double* __restrict__ Rs = ep.R + ep.offv[s];
+#pragma unroll
+      for (int j = 0; j < WC; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int c = mcol(j, e);
+          const double rc = (c < n) ? __ldg(Rs + c) : 0.0;
+#pragma unroll
+          for (int i = 0; i < WR; ++i) W[i][j][e] = mul_rn(W[i][j][e], rc);
+        }
+    }
     double* __restrict__ Og = bv.out + bv.offA[s];
     if (tile) {
-      const double* __restrict__ Rs = ep.R ? ep.R + ep.offv[s] : nullptr;
 #pragma unroll
       for (int i = 0; i < WR; ++i) {
-        const int r = grow(i);
+        const int r = mrow(i);
         if (r < n) {
 #pragma unroll
           for (int j = 0; j < WC; ++j)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int c = gcol(j, e);
-              if (c < n) Og[int64_t(r) * n + c] = Rs ? mul_rn(W[i][j][e], __ldg(Rs + c)) : W[i][j][e];
+              const int c = mcol(j, e);
+              if (c < n) Og[int64_t(r) * n + c] = W[i][j][e];
             }
         }
       }
     }
-    if (ep.C) {
-      // running totals of each row this CTA holds, from the B just written (L2):
-      // a warp takes 32 local rows and walks them in 32 x 32 tiles, loaded and
-      // stored coalesced through shared memory (the panel buffers, free now),
-      // each lane adding its own row left to right as the reference does.
-      // A cluster barrier first: warps of this CTA may still be reading the
-      // last step's panels in these buffers.
-      cluster_barrier<CL>();
+    cluster_wait<CL>();
+    if (EPI && ep.C) {
+      // Running totals of each row this CTA holds, left to right as the reference
+      // adds them, 16 columns at a time through shared memory (the panel buffers,
+      // free now).  Three pieces are under way: the warps that hold
+      // its two column blocks write one as B, a thread per row adds the 16 values
+      // of the one before to its total, and all warps store the one before that,
+      // 128 bytes a row; one barrier per piece.  Rows lie 16 apart, column k of
+      // row r at k ^ (r % 16): rows, columns and fragments all spread over the
+      // banks.  (Read back from L2 in 32 x 32 tiles by a warp per 32 rows, each
+      // add behind a load and a store, this took two thirds as long as the
+      // inverse: 8,192 cells of orders 20-200 4.99 ms in all, MATOM_NOW now.)
       double* __restrict__ Cg = ep.C + bv.offA[s];
-      constexpr int NG = (LP + 31) / 32;
-      if (tile && warp < NG) {
-        double* tl = sm + warp * (32 * 33);
-        auto row_of = [&](int lr) -> int {
-          return (lr < LP) ? ((((lr >> 3) * CL) + rank) * 8 + (lr & 7)) : n;
-        };
-        double total = 0.0;
-        for (int c0 = 0; c0 < n; c0 += 32) {
-          const int c = c0 + lane;
-#pragma unroll 8
-          for (int k = 0; k < 32; ++k) {
-            const int rk = row_of(warp * 32 + k);
-            tl[k * 33 + lane] = (rk < n && c < n) ? __ldcg(Og + int64_t(rk) * n + c) : 0.0;
+      constexpr int NG = (LP + 31) / 32;   // warps that add
+      auto piece = [&](int q) -> double* { return sm + (q % 3) * (LP * 16); };
+      const int np = (n + 15) / 16;
+      const int ra = 32 * warp + lane;     // the row this thread adds
+      double total = 0.0;
+      for (int q = 0; q < np + 2; ++q) {
+        if (tile && q < np) {
+          double* tl = piece(q);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int blk = 2 * q + h, jb = blk / WGC;
+            if (blk < nbe && blk - jb * WGC == wc) {
+#pragma unroll
+              for (int i = 0; i < WR; ++i) {
+                double v0 = W[i][0][0], v1 = W[i][0][1];
+#pragma unroll
+                for (int j = 1; j < WC; ++j)
+                  if (j == jb) {
+                    v0 = W[i][j][0];
+                    v1 = W[i][j][1];
+                  }
+                const int row = (wr + WGR * i) * 8 + pg;
+                double* d = tl + row * 16;
+                d[(8 * h + t) ^ (row & 15)] = v0;
+                d[(8 * h + t + 4) ^ (row & 15)] = v1;
+              }
+            }
           }
-          __syncwarp();
-          const int cm = min(32, n - c0);
-          for (int k = 0; k < cm; ++k) {
-            total = add_rn(total, tl[lane * 33 + k]);
-            tl[lane * 33 + k] = total;
-          }
-          __syncwarp();
-#pragma unroll 8
-          for (int k = 0; k < 32; ++k) {
-            const int rk = row_of(warp * 32 + k);
-            if (rk < n && c < n) Cg[int64_t(rk) * n + c] = tl[k * 33 + lane];
-          }
-          __syncwarp();
         }
+        if (tile && warp < NG && ra < LP && q >= 1 && q <= np) {
+          double* d = piece(q - 1) + ra * 16;
+          const int cm = n - 16 * (q - 1), sw = ra & 15;
+          double v[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] = d[k ^ sw];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            if (k < cm) total = add_rn(total, v[k]);
+            d[k ^ sw] = total;
+          }
+        }
+        if (tile && q >= 2) {
+          const double* tl = piece(q - 2);
+          const int c = lane & 15, cg = 16 * (q - 2) + c;
+#pragma unroll
+          for (int m = 0; m < (LP / 2 + NW - 1) / NW; ++m) {
+            const int row = 2 * (warp + NW * m) + (lane >> 4);
+            const int rk = (((row >> 3) * CL) + rank) * 8 + (row & 7);
+            if (row < LP && rk < n && cg < n) Cg[int64_t(rk) * n + cg] = tl[row * 16 + (c ^ (row & 15))];
+          }
+        }
+        __syncthreads();
       }
     }
     if (rank == 0 && tid == 0) {
       bv.status[s] = kOk;
       if (bv.diag) bv.diag[s] = 0;
     }
-    // the next item reuses the panel buffers: every CTA of the cluster is done
-    // with this one (including remote writes of its last pivot inverse)
-    cluster_barrier<CL>();
+    // the next item's first pivot inverse is written into every CTA's panel
+    // buffers: they are all done with their pieces (nothing to publish, so the
+    // arrival need not wait for the stores)
+    if (EPI && CL > 1 && ep.C) {
+      cluster_arrive_relaxed<CL>();
+      cluster_wait<CL>();
+    }
   }
 }
 

@@ -27,9 +27,14 @@ __device__ __forceinline__ int epi_count(int nsys, const EpiList& el) {
 }
 __device__ __forceinline__ int epi_system(int i, const EpiList& el) { return el.list ? el.list[i] : i; }
 
-// One CTA per system (grid-stride), one thread per row.  A singular system
-// (status != 0) gets B = 0 and C = 0: the reference's output of invert_matrix
-// is a zero-filled buffer that the failed call leaves untouched.
+// One CTA per system (grid-stride), a warp per 32 rows in 32 x 32 tiles: a tile's
+// 32 loads are in flight together, each row of it coalesced; the scaled tile is
+// stored as B and passes through shared memory to the lane of its row, which
+// adds it to the row's total; the totals leave the same way.  (A thread per row
+// straight from global memory, one 8-byte load at a time: 2,550 us for 2,048
+// cells of order 200, 470 us now.)  A singular system (status != 0) gets
+// B = 0 and C = 0: the reference's output of invert_matrix is a zero-filled
+// buffer that the failed call leaves untouched.
 __global__ void __launch_bounds__(128) matom_epilogue_kernel(int nsys, const int* __restrict__ n,
                                                              const int64_t* __restrict__ offA,
                                                              const int64_t* __restrict__ offv,
@@ -37,6 +42,9 @@ __global__ void __launch_bounds__(128) matom_epilogue_kernel(int nsys, const int
                                                              const double* __restrict__ R,
                                                              double* __restrict__ C,
                                                              const int* __restrict__ status, EpiList el) {
+  __shared__ double tiles[4][32 * 33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* tl = tiles[warp];
   const int count = epi_count(nsys, el);
   for (int i = blockIdx.x; i < count; i += gridDim.x) {
     const int s = epi_system(i, el);
@@ -45,14 +53,39 @@ __global__ void __launch_bounds__(128) matom_epilogue_kernel(int nsys, const int
     double* __restrict__ Bs = B + offA[s];
     double* __restrict__ Cs = C ? C + offA[s] : nullptr;
     const double* __restrict__ Rs = R + offv[s];
-    for (int r = threadIdx.x; r < ns; r += blockDim.x) {
-      double* __restrict__ brow = Bs + int64_t(r) * ns;
+    for (int r0 = 32 * warp; r0 < ns; r0 += 128) {
       double total = 0.0;
-      for (int c = 0; c < ns; ++c) {
-        const double b = ok ? mul_rn(brow[c], __ldg(Rs + c)) : 0.0;
-        brow[c] = b;
-        total = add_rn(total, b);
-        if (Cs) Cs[int64_t(r) * ns + c] = total;
+      for (int c0 = 0; c0 < ns; c0 += 32) {
+        const int c = c0 + lane;
+        double* __restrict__ bt = Bs + int64_t(r0) * ns + c;
+        const double rc = (c < ns) ? __ldg(Rs + c) : 0.0;
+        double v[32];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] = (ok && c < ns && r0 + k < ns) ? bt[int64_t(k) * ns] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+          v[k] = ok ? mul_rn(v[k], rc) : 0.0;
+          if (c < ns && r0 + k < ns) bt[int64_t(k) * ns] = v[k];
+        }
+        if (!Cs) continue;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) tl[k * 33 + lane] = v[k];
+        __syncwarp();
+        const int cm = min(32, ns - c0);
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] = tl[lane * 33 + k];
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+          if (k < cm) {
+            total = add_rn(total, v[k]);
+            tl[lane * 33 + k] = total;
+          }
+        __syncwarp();
+        double* __restrict__ ct = Cs + int64_t(r0) * ns + c;
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+          if (c < ns && r0 + k < ns) ct[int64_t(k) * ns] = tl[k * 33 + lane];
+        __syncwarp();
       }
     }
   }
