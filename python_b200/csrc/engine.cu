@@ -684,6 +684,27 @@ struct DevBuf {
   }
 };
 
+// Page-locked host memory that the GPU can address, grow-only up to a caller's bound.
+struct PinBuf {
+  void* ptr = nullptr;   // host address
+  void* dev = nullptr;   // the same memory, as the GPU addresses it
+  size_t bytes = 0;
+  int ensure(size_t want) {
+    if (want <= bytes) return 0;
+    release();
+    SS_CUDA(cudaHostAlloc(&ptr, want, cudaHostAllocMapped));
+    bytes = want;
+    SS_CUDA(cudaHostGetDevicePointer(&dev, ptr, 0));
+    return 0;
+  }
+  void release() {
+    if (ptr) cudaFreeHost(ptr);
+    ptr = dev = nullptr;
+    bytes = 0;
+  }
+  ~PinBuf() { release(); }
+};
+
 // A packed host batch split into chunks of consecutive systems, each with its
 // own plan, so that the copies of one chunk overlap the kernels of another.
 struct Pipeline {
@@ -747,6 +768,7 @@ struct Context {
   std::unordered_map<uint64_t, std::unique_ptr<Pipeline>> pipes;
   std::vector<uint64_t> pipe_order;
   DevBuf bA, bb, bx, bst;
+  PinBuf pin;   // one system of the drop-in calls, in and out
   DevBuf bR, bC, bOv, bN, bOa, bQs, bQl, bQz, bQt;   // macro-atom epilogue and draws
   DevBuf bIT, bI64, bID, bIL, bIS, bIA, bIB, bIX, bISt;   // ion rate-matrix assembly
   DevBuf bMT, bMD, bMN, bMR;                              // macro-atom jump-matrix assembly
@@ -766,6 +788,7 @@ struct Context {
     }
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
+    pin.release();
     device = -1;
   }
   int init() {
@@ -1902,6 +1925,32 @@ static int run_macro_pops(int ncell, int n, int nion, const int* ion_first, cons
   return 0;
 }
 
+// page-locked memory a thread's drop-in calls may hold (an inverse of order 361);
+// larger systems, whose kernels take milliseconds, go through pageable copies
+constexpr size_t kMaxPinBytes = size_t(2) << 20, kMinPinBytes = size_t(64) << 10;
+
+static int run_single_pageable(Context* c, sirocco_plan* p, int kind, const double* A, const double* b, int size,
+                               double* out, int* code) {
+  const size_t bytesA = sizeof(double) * size_t(size) * size;
+  const size_t bytesV = sizeof(double) * size_t(size);
+  int rc;
+  if ((rc = c->bA.ensure(bytesA)) || (rc = c->bst.ensure(sizeof(int)))) return rc;
+  if ((rc = c->bb.ensure(bytesV)) || (rc = c->bx.ensure(kind == kSolve ? bytesV : bytesA))) return rc;
+  double* dA = static_cast<double*>(c->bA.ptr);
+  double* db = static_cast<double*>(c->bb.ptr);
+  double* dx = static_cast<double*>(c->bx.ptr);
+  int* dst = static_cast<int*>(c->bst.ptr);
+  SS_CUDA(cudaMemcpyAsync(dA, A, bytesA, cudaMemcpyHostToDevice, c->stream));
+  if (kind == kSolve) SS_CUDA(cudaMemcpyAsync(db, b, bytesV, cudaMemcpyHostToDevice, c->stream));
+  rc = plan_run(p, dA, db, dx, dst, nullptr, c->stream);
+  if (rc) return rc;
+  SS_CUDA(cudaMemcpyAsync(code, dst, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  SS_CUDA(cudaStreamSynchronize(c->stream));
+  const bool write = (kind == kSolve) ? (*code != kSolveSingular) : (*code == kOk);
+  if (write) SS_CUDA(cudaMemcpy(out, dx, kind == kSolve ? bytesV : bytesA, cudaMemcpyDeviceToHost));
+  return 0;
+}
+
 // single system through the host path, honouring the reference's "output
 // untouched on a singular matrix" behaviour
 static int run_single(int kind, double* A, const double* b, int size, double* out, int* code) {
@@ -1917,22 +1966,37 @@ static int run_single(int kind, double* A, const double* b, int size, double* ou
   sirocco_plan* p = nullptr;
   rc = c->get_plan(kind, 1, nn, oa, kind == kSolve ? ov : nullptr, SIROCCO_FP64, &p);
   if (rc) return rc;
-  const size_t bytesA = sizeof(double) * size_t(size) * size;
-  const size_t bytesV = sizeof(double) * size_t(size);
-  if ((rc = c->bA.ensure(bytesA)) || (rc = c->bst.ensure(sizeof(int)))) return rc;
-  if ((rc = c->bb.ensure(bytesV)) || (rc = c->bx.ensure(kind == kSolve ? bytesV : bytesA))) return rc;
-  double* dA = static_cast<double*>(c->bA.ptr);
-  double* db = static_cast<double*>(c->bb.ptr);
-  double* dx = static_cast<double*>(c->bx.ptr);
-  int* dst = static_cast<int*>(c->bst.ptr);
-  SS_CUDA(cudaMemcpyAsync(dA, A, bytesA, cudaMemcpyHostToDevice, c->stream));
-  if (kind == kSolve) SS_CUDA(cudaMemcpyAsync(db, b, bytesV, cudaMemcpyHostToDevice, c->stream));
-  rc = plan_run(p, dA, db, dx, dst, nullptr, c->stream);
+  const size_t nA = size_t(size) * size, nV = kind == kSolve ? size_t(size) : 0, nO = kind == kSolve ? nV : nA;
+  // [A | b | out | code] in page-locked memory: a system that a warp solves is
+  // read and answered by the kernel where it lies (its matrix is read once, and
+  // the way over the bus is shorter than one copy's launch); a larger one is
+  // copied, in one piece each way.  One wait per call.  (Pageable copies, each
+  // waited for by itself: 64 us a solve of order 27, with the same kernel 56 us;
+  // 34 us now.)
+  const size_t total = sizeof(double) * (nA + nV + nO + 1);
+  if (total > kMaxPinBytes) return run_single_pageable(c, p, kind, A, b, size, out, code);
+  if ((rc = c->pin.ensure(std::max(total, kMinPinBytes)))) return rc;
+  double* h = static_cast<double*>(c->pin.ptr);
+  double* hout = h + nA + nV;
+  int* hcode = reinterpret_cast<int*>(hout + nO);
+  std::memcpy(h, A, sizeof(double) * nA);
+  if (kind == kSolve) std::memcpy(h + nA, b, sizeof(double) * nV);
+  double* d = static_cast<double*>(c->pin.dev);
+  const bool in_place = size <= kMaxSmallN;
+  if (!in_place) {
+    if ((rc = c->bA.ensure(total))) return rc;
+    d = static_cast<double*>(c->bA.ptr);
+    SS_CUDA(cudaMemcpyAsync(d, h, sizeof(double) * (nA + nV), cudaMemcpyHostToDevice, c->stream));
+  }
+  double* dout = d + nA + nV;
+  rc = plan_run(p, d, d + nA, dout, reinterpret_cast<int*>(dout + nO), nullptr, c->stream);
   if (rc) return rc;
-  SS_CUDA(cudaMemcpyAsync(code, dst, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if (!in_place)
+    SS_CUDA(cudaMemcpyAsync(hout, dout, sizeof(double) * (nO + 1), cudaMemcpyDeviceToHost, c->stream));
   SS_CUDA(cudaStreamSynchronize(c->stream));
+  *code = *hcode;
   const bool write = (kind == kSolve) ? (*code != kSolveSingular) : (*code == kOk);
-  if (write) SS_CUDA(cudaMemcpy(out, dx, kind == kSolve ? bytesV : bytesA, cudaMemcpyDeviceToHost));
+  if (write) std::memcpy(out, hout, sizeof(double) * nO);
   return 0;
 }
 
