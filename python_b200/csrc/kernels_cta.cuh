@@ -223,7 +223,7 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
             }
           }
           // reciprocal of the thread's own candidate, overlapping the reduction
-          const double rb = __drcp_rn(vb);
+          const double rb = rcp_markstein(vb);
           const unsigned hi = unsigned(kb >> 32), lo = unsigned(kb);
           const unsigned mh = __reduce_max_sync(FULL, hi);
           const unsigned ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
@@ -280,6 +280,7 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
             rinv = __shfl_sync(FULL, rb, pl);   // = fl(1/u_jj), correctly rounded
           }
           const double ujj = pv[0];
+          if (!rcp_covers(ujj)) rinv = rcp_outline(ujj);   // the same on every lane
           if (__any_sync(FULL, ujj == 0.0)) { sing = true; break; }
           if (KIND == kInvert && t == 0 && isinf(ujj)) flags[1] = 1;
           double lrow[RPL];
@@ -472,6 +473,9 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
           rhs[r] = v;
         }
       }
+      // A solve's rows are taken in position order from the first one left, so
+      // that rows already chosen cost nothing; an inverse updates every row.
+      const int left0 = j0 + B;
       if (!GM) {
         // Shared memory: column by column.  The panel's own columns are
         // skipped, a solve skips its L columns too, and the inverse's columns
@@ -480,15 +484,22 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
         // multiply-subtract with k ascending.
 #pragma unroll 1
         for (int rg = 0; rg < RB; rg += RG) {
+          if (KIND == kSolve && left0 + TGR * rg >= n) break;
           int row[RG], sw[RG];
           bool keep[RG];
           double mk[B][RG];
 #pragma unroll
           for (int u = 0; u < RG; ++u) {
-            row[u] = tr + TGR * (rg + u);
+            const int at = tr + TGR * (rg + u);
+            if (KIND == kSolve) {
+              keep[u] = left0 + at < n;
+              row[u] = keep[u] ? perm[left0 + at] : 0;
+            } else {
+              row[u] = at;
+              const int p = ps_s[at];
+              keep[u] = at < n && (p < j0 || p >= j0 + nb);
+            }
             sw[u] = cta_swz(row[u]);
-            const int p = ps_s[row[u]];
-            keep[u] = row[u] < n && (p < j0 || p >= j0 + nb) && (KIND == kInvert || p >= j0 + B);
 #pragma unroll
             for (int k = 0; k < B; ++k) mk[k][u] = Mm[row[u] * MS + k];
           }
@@ -523,13 +534,20 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
         // with k ascending except on tiles wholly left of the panel.
 #pragma unroll 1
         for (int rg = 0; rg < RB; rg += RG) {
+          if (KIND == kSolve && left0 + TGR * rg >= n) break;
           int row[RG];
           bool keep[RG];
 #pragma unroll
           for (int u = 0; u < RG; ++u) {
-            row[u] = tr + TGR * (rg + u);
-            const int p = ps_s[row[u]];
-            keep[u] = row[u] < n && (p < j0 || p >= j0 + nb) && (KIND == kInvert || p >= j0 + B);
+            const int at = tr + TGR * (rg + u);
+            if (KIND == kSolve) {
+              keep[u] = left0 + at < n;
+              row[u] = keep[u] ? perm[left0 + at] : 0;
+            } else {
+              row[u] = at;
+              const int p = ps_s[at];
+              keep[u] = at < n && (p < j0 || p >= j0 + nb);
+            }
           }
 #pragma unroll 1
           for (int cg = 0; cg < CB; cg += CC) {

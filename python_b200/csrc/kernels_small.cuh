@@ -245,20 +245,6 @@ __device__ __noinline__ PivotChoice small_pivot_general(double v, bool elig, int
   return r;
 }
 
-// fl(1 / d) for d in [2^-1021, 2^1021) whose significand is not all ones: the
-// hardware's approximation (2^-20), one cubic Newton-Raphson step (below one ulp)
-// and Markstein's correcting step, which rounds correctly from there (P.
-// Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990).  Branch-free, so that it overlaps a reduction: __drcp_rn in
-// its place cost 300 cycles of a pivot step's 815.
-__device__ __forceinline__ double rcp_markstein(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-d, y, 1.0);
-  y = fma(fma(e, e, e), y, y);
-  return fma(fma(-d, y, 1.0), y, y);
-}
-
 // fl(u / d) from r = fl(1 / d) for a quotient well inside the range: Markstein's
 // division (two remainders, the second from a quotient within one ulp, round
 // correctly).  far keeps the largest distance from the range where that holds:
