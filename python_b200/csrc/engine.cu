@@ -94,6 +94,15 @@ static const int kCtaP[] = {
 };
 constexpr int kCtaClasses = int(sizeof(kCtaP) / sizeof(kCtaP[0]));
 
+// largest orders of the classes of many solves (cta_solve_classes.inc)
+static const int kCtaSolveN[] = {
+#define SS_CTA_SOLVE_CLASS(I, LIM, P, NT, RG, CC, PW, GM, MINB) LIM,
+#include "cta_solve_classes.inc"
+#undef SS_CTA_SOLVE_CLASS
+};
+constexpr int kCtaSolveClasses = int(sizeof(kCtaSolveN) / sizeof(kCtaSolveN[0]));
+constexpr int kCtaTables = kCtaClasses > kCtaSolveClasses ? kCtaClasses : kCtaSolveClasses;
+
 // padded orders of the certified Gauss-Jordan classes (cgj_classes.inc)
 static const int kCgjP[] = {
 #define SS_CGJ_CLASS(I, P, WGR, WGC, CL, MINB, ST) P,
@@ -115,6 +124,11 @@ static int small_class(int n) {
 static int cta_class(int n) {
   for (int i = 0; i < kCtaClasses; ++i)
     if (n <= kCtaP[i]) return i;
+  return -1;
+}
+static int cta_solve_class(int n) {
+  for (int i = 0; i < kCtaSolveClasses; ++i)
+    if (n <= kCtaSolveN[i]) return i;
   return -1;
 }
 static int cgj_class(int n) {
@@ -144,27 +158,40 @@ static KernelSpec small_spec(int cls, int mode) {
   return k;
 }
 
-template <int KIND>
-static KernelSpec cta_spec(int cls) {
+template <int KIND, int P, int NT, int RG, int CC, int PW, bool GM, int MINB>
+static KernelSpec cta_shape_spec() {
+  using Sh = CtaShape<KIND, P, NT, RG, CC, PW, GM, MINB>;
   KernelSpec k;
-#define SS_CTA_CLASS(I, P, NT, RG, CC, PW, GM, MINB)                                    \
-  case I: {                                                                             \
-    using Sh = CtaShape<KIND, P, NT, RG, CC, PW, GM, MINB>;                             \
-    k.fn = reinterpret_cast<const void*>(&cta_exact_kernel<KIND, P, NT, RG, CC, PW, GM, MINB>); \
-    k.threads = NT;                                                                     \
-    k.dyn_smem = Sh::dyn_smem;                                                          \
-    k.work_slab = Sh::slab;                                                             \
-    break;                                                                              \
+  k.fn = reinterpret_cast<const void*>(&cta_exact_kernel<KIND, P, NT, RG, CC, PW, GM, MINB>);
+  k.threads = NT;
+  k.dyn_smem = Sh::dyn_smem;
+  k.work_slab = Sh::slab;
+  return k;
+}
+
+// the class tables: cta_classes.inc, inverses measured per class by
+// python_b200/autotune.py (shared memory for the smallest orders, a global
+// workspace slab above them, where more CTAs per SM, more pivot chains in flight,
+// beat the faster memory), and for many solves cta_solve_classes.inc
+static KernelSpec cta_spec(int kind, int cls, bool many_solves) {
+  if (kind == kSolve && many_solves) {
+#define SS_CTA_SOLVE_CLASS(I, LIM, P, NT, RG, CC, PW, GM, MINB) \
+  case I: return cta_shape_spec<kSolve, P, NT, RG, CC, PW, GM, MINB>();
+    switch (cls) {
+#include "cta_solve_classes.inc"
+      default: return KernelSpec();
+    }
+#undef SS_CTA_SOLVE_CLASS
   }
-  // the class table, measured per class by python_b200/autotune.py: shared
-  // memory for the smallest orders, a global workspace slab above them, where
-  // more CTAs per SM (more pivot chains in flight) beat the faster memory
+#define SS_CTA_CLASS(I, P, NT, RG, CC, PW, GM, MINB)                           \
+  case I:                                                                      \
+    return kind == kSolve ? cta_shape_spec<kSolve, P, NT, RG, CC, PW, GM, MINB>() \
+                          : cta_shape_spec<kInvert, P, NT, RG, CC, PW, GM, MINB>();
   switch (cls) {
 #include "cta_classes.inc"
-    default: break;
+    default: return KernelSpec();
   }
 #undef SS_CTA_CLASS
-  return k;
 }
 
 static KernelSpec cgj_spec(int cls) {
@@ -383,7 +410,7 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
   // Certified inverses (SIROCCO_FAST) go to the Gauss-Jordan classes; each also
   // has a place in the fallback list of its exact class (small or CTA family).
   const bool cert = (kind == kInvert && mode == SIROCCO_FAST);
-  std::vector<int> small_n[kMaxSmallN + 1], small_l[kSmallClasses], cta_l[kCtaClasses], glob_l, cgj_l[kCgjClasses],
+  std::vector<int> small_n[kMaxSmallN + 1], small_l[kSmallClasses], cta_l[kCtaTables], glob_l, cgj_l[kCgjClasses],
       cgjl_l;
   int small_fb[kSmallClasses] = {}, cta_fb[kCtaClasses] = {};
   for (int s = 0; s < nsys; ++s) {
@@ -415,6 +442,28 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
   for (int ns = 1; ns <= kMaxSmallN; ++ns) {
     std::vector<int>& l = small_l[small_class(ns)];
     l.insert(l.end(), small_n[ns].begin(), small_n[ns].end());
+  }
+  // Solves of the CTA family: with no more systems than the inverse's shapes
+  // run at once, those shapes (more threads, the shorter single solve); beyond
+  // that, the solves' own, with more systems in flight.  (592 of order 60: 89 us
+  // against 108; 1,184: 174 against 130.  296 of order 180: 574 against 611;
+  // 1,184: 2,226 against 1,866.)
+  bool many = false;
+  if (kind == kSolve) {
+    double rounds = 0.0;
+    for (int c = 0; c < kCtaClasses; ++c)
+      if (!cta_l[c].empty()) {
+        KernelSpec k = cta_spec(kSolve, c, false);
+        if (int rc = finish_spec(k)) return rc;
+        rounds += double(cta_l[c].size()) / k.max_ctas;
+      }
+    many = rounds > 1.0;
+    if (many) {
+      std::vector<int> again[kCtaTables];
+      for (auto& l : cta_l)
+        for (int s : l) again[cta_solve_class(n[s])].push_back(s);
+      for (int c = 0; c < kCtaTables; ++c) cta_l[c].swap(again[c]);
+    }
   }
   // fallback lists: one per exact class that certified systems belong to
   int small_fbi[kSmallClasses], cta_fbi[kCtaClasses];
@@ -466,7 +515,7 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
       b.q = p->nq++;
     }
     else if (fam == kFamSmall) b.spec = (kind == kSolve) ? small_spec<kSolve>(cls, mode) : small_spec<kInvert>(cls, mode);
-    else if (fam == kFamCta) b.spec = (kind == kSolve) ? cta_spec<kSolve>(cls) : cta_spec<kInvert>(cls);
+    else if (fam == kFamCta) b.spec = cta_spec(kind, cls, many);
     else b.spec = (kind == kSolve) ? global_spec<kSolve>(cls) : global_spec<kInvert>(cls);
     int rc = finish_spec(b.spec);
     if (rc) return rc;
@@ -494,7 +543,7 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
   if ((rc = add_bucket(kFamCgjL, 0, cgjl_l))) return rc;
   for (int c = kCgjClasses - 1; c >= 0; --c)
     if ((rc = add_bucket(kFamCgj, c, cgj_l[c]))) return rc;
-  for (int c = kCtaClasses - 1; c >= 0; --c)
+  for (int c = kCtaTables - 1; c >= 0; --c)
     if ((rc = add_bucket(kFamCta, c, cta_l[c]))) return rc;
   for (int c = kSmallClasses - 1; c >= 0; --c)
     if ((rc = add_bucket(kFamSmall, c, small_l[c]))) return rc;

@@ -71,9 +71,10 @@ struct CtaShape {
   static constexpr int off_V = off_Mm + P * MS;
   static constexpr int off_r = off_V + B * P;
   static constexpr int off_pb = off_r + B; // pivot-row exchange of a multi-warp panel
-  // solves: the right-hand side rides along by row, its pivot values of a panel beside it
+  // solves: the right-hand side rides along by row, its pivot values of a panel
+  // beside it, and the reciprocals of the pivots are kept
   static constexpr int off_rhs = off_pb + B + 2;
-  static constexpr int n_dbl = off_rhs + (KIND == kSolve ? P + B : 0);
+  static constexpr int n_dbl = off_rhs + (KIND == kSolve ? 2 * P + B : 0);
   static constexpr int n_int = 2 * P + 4 + 4 * PW;
   static constexpr size_t dyn_smem = size_t(n_dbl) * 8 + size_t(n_int) * 4;
   static constexpr int by_smem = int(kSmemPerSm / (dyn_smem + 1024));
@@ -108,6 +109,7 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
   int* flags = perm + P;                   // [0] singular, [1] an infinite pivot, [2] first failing row of a solve
   double* rhs = dsm + Sh::off_rhs;         // solves: [P] right-hand side by row, [B] the panel's pivot values
   double* vrhs = rhs + P;
+  double* rdiag = vrhs + B;                // solves: [P] fl(1/u_jj) by position, 0 where not known to be rounded so
   unsigned* cand = reinterpret_cast<unsigned*>(flags + 4);   // [PW][4] per-warp pivot candidates
 
   const int t = threadIdx.x;
@@ -317,6 +319,7 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
           drinv = rinv;
           dk = k;
           if (t == 0) rinv_s[k] = rinv;
+          if (KIND == kSolve && t == 0) rdiag[j] = rcp_covers(ujj) ? rinv : 0.0;
 #pragma unroll
           for (int i = 0; i < RPL; ++i) {
             const double first = pr[i][0];
@@ -473,8 +476,10 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
           rhs[r] = v;
         }
       }
-      // A solve's rows are taken in position order from the first one left, so
-      // that rows already chosen cost nothing; an inverse updates every row.
+      // In the workspace a solve's rows are taken in position order from the first
+      // one left, so that rows already chosen cost nothing (in shared memory that
+      // order costs more in bank conflicts than it saves); an inverse updates
+      // every row.
       const int left0 = j0 + B;
       if (!GM) {
         // Shared memory: column by column.  The panel's own columns are
@@ -484,22 +489,15 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
         // multiply-subtract with k ascending.
 #pragma unroll 1
         for (int rg = 0; rg < RB; rg += RG) {
-          if (KIND == kSolve && left0 + TGR * rg >= n) break;
           int row[RG], sw[RG];
           bool keep[RG];
           double mk[B][RG];
 #pragma unroll
           for (int u = 0; u < RG; ++u) {
-            const int at = tr + TGR * (rg + u);
-            if (KIND == kSolve) {
-              keep[u] = left0 + at < n;
-              row[u] = keep[u] ? perm[left0 + at] : 0;
-            } else {
-              row[u] = at;
-              const int p = ps_s[at];
-              keep[u] = at < n && (p < j0 || p >= j0 + nb);
-            }
+            row[u] = tr + TGR * (rg + u);
             sw[u] = cta_swz(row[u]);
+            const int p = ps_s[row[u]];
+            keep[u] = row[u] < n && (p < j0 || p >= j0 + nb) && (KIND == kInvert || p >= j0 + B);
 #pragma unroll
             for (int k = 0; k < B; ++k) mk[k][u] = Mm[row[u] * MS + k];
           }
@@ -637,64 +635,73 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
       // the factorisation): x_i = (y_i - U_i,i+1 x_i+1 - U_i,i+2 x_i+2 - ...) /
       // U_ii.  Each sum starts with the x just found, so GSL's order is one
       // chain of n^2 / 2 dependent subtractions; everything else is kept off it.
-      // Warp 0 holds row i's products U_ik x_k, k >= i + 2, in shared memory
-      // (formed by its 32 lanes while row i + 1's chain ran; zeros pad both
-      // ends of the range, and u - 0 = u), every lane runs the chain from
-      // broadcast 16-byte loads, and row i - 1's entries are on their way
-      // meanwhile.  It was one lane walking U, each step waiting on its load:
-      // n = 204 alone on an SM took 1.1 ms in all, and 4,096 systems of orders
-      // 33-200 8.02 ms (4.99 ms now).
-      double* Pb = Vs;                     // [P + 8] products of the current row
+      // Warp 0 holds row i's products U_ik x_k, k >= i + 2, in shared memory, formed
+      // by its 32 lanes a row ahead from entries loaded a row before that (zeros
+      // pad both ends of the range, and u - 0 = u); every lane runs the chain from
+      // broadcast 16-byte loads, and the quotients are div_markstein's.  It was one
+      // lane walking U, each step waiting on its load: n = 204 alone on an SM took
+      // 1.1 ms in all, and 4,096 systems of orders 33-200 8.0 ms (3.5 ms now).
+      double* Pb = Vs;                     // [2][P] products of a row, by its parity
       double* xs = Vs + 4 * P;             // [P] solution, clear of the check's tiles below
       const int64_t ov = bv.offv[s];
       if (wid == 0) {
-        const int r = perm[n - 1];
-        if (wl < 8) Pb[(n & ~7) + wl] = 0.0;
+        constexpr int MU = (P + 31) / 32 < 8 ? (P + 31) / 32 : 8;   // a lane's entries of a row (of 256 columns)
+        const int n8 = (n + 7) & ~7;
+        if (wl < 8 && (n & ~7) + wl < P) Pb[(n & ~7) + wl] = Pb[P + (n & ~7) + wl] = 0.0;
         __syncwarp();
-        double y = rhs[r], d = M[r * P + ((n - 1) ^ cta_swz(r))], e = 0.0, xp = 0.0;
+        const int r = perm[n - 1];
+        double y = rhs[r], d = M[r * P + ((n - 1) ^ cta_swz(r))], e = 0.0, xp = 0.0, ri = rdiag[n - 1];
+        double un[MU];                     // row i - 1's entries, up to 256 columns from its first product
+#pragma unroll
+        for (int m = 0; m < MU; ++m) un[m] = 0.0;
         for (int i = n - 1; i >= 0; --i) {
-          const int ip = (i > 0) ? i - 1 : 0;
+          const int ip = (i > 0) ? i - 1 : 0, iq = (i > 1) ? i - 2 : 0;
           const int rn = perm[ip], swn = cta_swz(rn);
           const double* Un = M + rn * P;
-          const double yn = rhs[rn], dn = Un[ip ^ swn], en = Un[i ^ swn];
+          const double yn = rhs[rn], dn = Un[ip ^ swn], en = Un[i ^ swn], rin = rdiag[ip];
+          // row i - 1's products, k >= i + 1
+          double* Pn = Pb + ((i + 1) & 1) * P;
+          const int kn = (i + 1) & ~7;
+#pragma unroll
+          for (int m = 0; m < MU; ++m) {
+            const int k = kn + wl + 32 * m;
+            if (k < n8) Pn[k] = (k >= i + 1 && k < n) ? mul_rn(un[m], xs[k]) : 0.0;
+          }
+          if (P > 256)
+            for (int k = kn + 256 + wl; k < n8; k += 32) Pn[k] = (k < n) ? mul_rn(Un[k ^ swn], xs[k]) : 0.0;
+          // row i - 2's entries, k >= i
+          const int r2 = perm[iq], sw2 = cta_swz(r2);
+          const int k2 = i & ~7;
+#pragma unroll
+          for (int m = 0; m < MU; ++m) {
+            const int k = k2 + wl + 32 * m;
+            un[m] = (k >= i && k < n) ? M[r2 * P + (k ^ sw2)] : 0.0;
+          }
+          // row i's chain
           double u = y;
           if (i + 1 < n) u = sub_rn(u, mul_rn(e, xp));
-          // in pieces of 256 columns: row i - 1's entries loaded, row i's chain, then
-          // row i - 1's products over the ones just used
-          const int kn = i + 1;            // first product of row i - 1
-          for (int kc = kn & ~7; kc < n; kc += 256) {
-            double un[8];
-#pragma unroll
-            for (int m = 0; m < 8; ++m) {
-              const int k = kc + wl + 32 * m;
-              un[m] = (k >= kn && k < n) ? Un[k ^ swn] : 0.0;
-            }
-            const int ke = min(n, kc + 256);
-            for (int k = max(kc, (i + 2) & ~7); k < ke; k += 8) {
-              const double2* p2 = reinterpret_cast<const double2*>(Pb + k);
-              const double2 p0 = p2[0], p1 = p2[1], p3 = p2[2], p4 = p2[3];
-              u = sub_rn(u, p0.x);
-              u = sub_rn(u, p0.y);
-              u = sub_rn(u, p1.x);
-              u = sub_rn(u, p1.y);
-              u = sub_rn(u, p3.x);
-              u = sub_rn(u, p3.y);
-              u = sub_rn(u, p4.x);
-              u = sub_rn(u, p4.y);
-            }
-            __syncwarp();
-#pragma unroll
-            for (int m = 0; m < 8; ++m) {
-              const int k = kc + wl + 32 * m;
-              if (k < ((n + 7) & ~7)) Pb[k] = (k >= kn && k < n) ? mul_rn(un[m], xs[k]) : 0.0;
-            }
+          const double* Pi = Pb + (i & 1) * P;
+          for (int k = (i + 2) & ~7; k < n; k += 8) {
+            const double2* p2 = reinterpret_cast<const double2*>(Pi + k);
+            const double2 p0 = p2[0], p1 = p2[1], p3 = p2[2], p4 = p2[3];
+            u = sub_rn(u, p0.x);
+            u = sub_rn(u, p0.y);
+            u = sub_rn(u, p1.x);
+            u = sub_rn(u, p1.y);
+            u = sub_rn(u, p3.x);
+            u = sub_rn(u, p3.y);
+            u = sub_rn(u, p4.x);
+            u = sub_rn(u, p4.y);
           }
-          xp = div_rn(u, d);
+          unsigned far = 0u;
+          xp = div_markstein(u, d, ri, far);
+          if (far >= kDivFar) xp = div_outline(u, d);   // the same on every lane
           if (wl == 0) xs[i] = xp;
           __syncwarp();
           y = yn;
           d = dn;
           e = en;
+          ri = rin;
         }
         for (int i = wl; i < n; i += 32) bv.out[ov + i] = xs[i];
       }

@@ -245,23 +245,6 @@ __device__ __noinline__ PivotChoice small_pivot_general(double v, bool elig, int
   return r;
 }
 
-// fl(u / d) from r = fl(1 / d) for a quotient well inside the range: Markstein's
-// division (two remainders, the second from a quotient within one ulp, round
-// correctly).  far keeps the largest distance from the range where that holds:
-// kDivFar or more when some |u| or quotient left 2^+-900 (u = 0 stays inside:
-// its quotient is u r), so that a remainder may have been subnormal.
-constexpr unsigned kDivFar = 0x70800000u;
-__device__ __forceinline__ double div_markstein(double u, double d, double r, unsigned& far) {
-  const double q0 = u * r;
-  const double q1 = fma(fma(-q0, d, u), r, q0);
-  const double q = fma(fma(-q1, d, u), r, q1);
-  const unsigned hu = (unsigned(__double2hiint(u)) & 0x7fffffffu) - 0x07b00000u;
-  const unsigned hq = (unsigned(__double2hiint(q)) & 0x7fffffffu) - 0x07b00000u;
-  const bool zero = (u == 0.0) && r != 0.0;
-  far = max(far, zero ? 0u : max(hu, hq));
-  return zero ? q0 : q;
-}
-
 // The upper sweep by divisions, one lane of each group walking U as GSL does: for
 // systems whose quotients div_markstein may not round correctly.  Returns x_lane.
 template <int NP, int G>

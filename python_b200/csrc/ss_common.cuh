@@ -101,6 +101,25 @@ __device__ __forceinline__ double rcp_markstein(double d) {
   return fma(fma(-d, y, 1.0), y, y);
 }
 
+// fl(u / d) from r = fl(1 / d) for a quotient well inside the range: Markstein's
+// division (two remainders, the second from a quotient within one ulp, round
+// correctly).  far keeps the largest distance from the range where that holds:
+// kDivFar or more when some |u| or quotient left 2^+-900 (u = 0 stays inside:
+// its quotient is u r), so that a remainder may have been subnormal.
+constexpr unsigned kDivFar = 0x70800000u;
+__device__ __forceinline__ double div_markstein(double u, double d, double r, unsigned& far) {
+  const double q0 = u * r;
+  const double q1 = fma(fma(-q0, d, u), r, q0);
+  const double q = fma(fma(-q1, d, u), r, q1);
+  const unsigned hu = (unsigned(__double2hiint(u)) & 0x7fffffffu) - 0x07b00000u;
+  const unsigned hq = (unsigned(__double2hiint(q)) & 0x7fffffffu) - 0x07b00000u;
+  const bool zero = (u == 0.0) && r != 0.0;
+  far = max(far, zero ? 0u : max(hu, hq));
+  return zero ? q0 : q;
+}
+
+__device__ __noinline__ double div_outline(double u, double d) { return div_rn(u, d); }
+
 // Whether rcp_markstein(d) is fl(1 / d) for certain, and fl(1 / d) where it is not.
 __device__ __forceinline__ bool rcp_covers(double d) {
   return (unsigned(__double2hiint(d)) & 0x7fffffffu) - 0x00200000u < 0x7fa00000u && __double2loint(d) != -1;

@@ -8,8 +8,8 @@ from oracle import oracle
 from python_b200 import workloads as wl
 from helpers import same_values
 
-ORDERS = (33, 39, 40, 41, 47, 48, 49, 63, 64, 65, 95, 96, 97, 127, 128, 129, 160, 161, 192, 193, 207, 208, 209, 223,
-          224, 225, 255, 256, 257, 263, 264, 320, 321, 511, 512, 513)
+ORDERS = (33, 39, 40, 41, 47, 48, 49, 63, 64, 65, 79, 80, 81, 95, 96, 97, 127, 128, 129, 160, 161, 192, 193, 207, 208, 209, 223,
+          224, 225, 255, 256, 257, 263, 264, 320, 321, 384, 385, 448, 449, 511, 512, 513)
 
 
 @pytest.mark.gpu
