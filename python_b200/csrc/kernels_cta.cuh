@@ -703,7 +703,6 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
           e = en;
           ri = rin;
         }
-        for (int i = wl; i < n; i += 32) bv.out[ov + i] = xs[i];
       }
       __syncthreads();
       // residual check on the original A (matrix_cpu.c:155-187), first failing
@@ -752,6 +751,8 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
         __syncwarp();
       }
       __syncthreads();
+      // x leaves last: the caller's x may be its b, which the check reads
+      for (int i = t; i < n; i += NT) bv.out[ov + i] = xs[i];
       if (t == 0) {
         bv.status[s] = (flags[2] == 0x7fffffff) ? kOk : (flags[2] & 3);
         if (bv.diag) bv.diag[s] = kDiagExact;
