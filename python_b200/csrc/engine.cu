@@ -1613,7 +1613,11 @@ template <int NPM>
 static int launch_ion_lock(Context* c, const IonAsmView& v, const IonLockView& lv, int warps) {
   const size_t smem = ion_lock_smem<NPM>(warps, v.nions);
   const auto fn = &ion_lockstep_kernel<NPM>;
-  SS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  // The limit belongs to the function, which every host thread shares: always the
+  // most that any table takes, so that no thread lowers it under another's launch.
+  constexpr size_t most = ion_lock_smem<NPM>(kIonLockWarps, kIonLockMaxIons);
+  static_assert(most <= 232448, "one CTA's shared memory");
+  SS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)));
   int nb = 0;
   SS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * warps, smem));
   fn<<<std::min(lv.ncell, std::max(1, nb) * c->num_sms), 32 * warps, smem, c->stream>>>(v, lv);

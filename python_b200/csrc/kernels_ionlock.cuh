@@ -39,7 +39,7 @@ constexpr double kLockFracError = 0.03;       // python.h:1212
 // dynamic shared memory: a solve's scratch per warp, then the cell's new
 // populations and their terms of n_e
 template <int NPM>
-size_t ion_lock_smem(int warps, int nions) {
+constexpr size_t ion_lock_smem(int warps, int nions) {
   return sizeof(SmallSmem<NPM>) * size_t(warps) + sizeof(double) * 2 * size_t(nions);
 }
 
