@@ -159,8 +159,14 @@ struct CgjShape {
   static_assert(buf % 2 == 0 && off_dg % 2 == 0, "16-byte aligned buffers");
   static_assert(!STAGE || LB <= 32, "one lane of the pivot warp issues each block's copy");
   static_assert(dyn_smem <= 232448, "one CTA's shared memory");
-  static_assert(3 * LP * 16 <= off_dg && (LP + 31) / 32 <= NW,
+  // Running-total pieces of the macro-atom epilogue, [LP][16] each, over the panel
+  // buffers.  On a cluster they leave D^-1 and Dnext of both buffers alone: a peer
+  // writes the next matrix's first D^-1 there while this CTA is still at its pieces.
+  static constexpr int off_pc1 = 16 * LP;
+  static constexpr int off_pc2 = (CL > 1) ? buf : 2 * 16 * LP;
+  static_assert(off_pc2 + 16 * LP <= off_dg && (LP + 31) / 32 <= NW,
                 "three running-total pieces fit the panel buffers, one tile warp per 32 rows");
+  static_assert(CL == 1 || 2 * 16 * LP <= off_Dinv, "a cluster's pieces lie below D^-1 in either panel buffer");
 };
 
 __device__ __forceinline__ unsigned cluster_rank() {
@@ -181,10 +187,6 @@ __device__ __forceinline__ void cluster_barrier() {
 template <int CL>
 __device__ __forceinline__ void cluster_arrive() {
   if (CL > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-}
-template <int CL>
-__device__ __forceinline__ void cluster_arrive_relaxed() {
-  if (CL > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
 }
 template <int CL>
 __device__ __forceinline__ void cluster_wait() {
@@ -888,7 +890,10 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
       // inverse: 8,192 cells of orders 20-200 4.99 ms in all, 3.94 now.)
       double* __restrict__ Cg = ep.C + bv.offA[s];
       constexpr int NG = (LP + 31) / 32;   // warps that add
-      auto piece = [&](int q) -> double* { return sm + (q % 3) * (LP * 16); };
+      auto piece = [&](int q) -> double* {
+        const int m = q % 3;
+        return sm + (m == 0 ? 0 : m == 1 ? S::off_pc1 : S::off_pc2);
+      };
       const int np = (n + 15) / 16;
       const int ra = 32 * warp + lane;     // the row this thread adds
       double total = 0.0;
@@ -945,13 +950,9 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
       bv.status[s] = kOk;
       if (bv.diag) bv.diag[s] = 0;
     }
-    // the next item's first pivot inverse is written into every CTA's panel
-    // buffers: they are all done with their pieces (nothing to publish, so the
-    // arrival need not wait for the stores)
-    if (EPI && CL > 1 && ep.C) {
-      cluster_arrive_relaxed<CL>();
-      cluster_wait<CL>();
-    }
+    // No barrier between a cluster's CTAs here: until the next certificate's, all
+    // that a peer writes into this CTA is the next matrix's first D^-1, which was
+    // last read before the arrival above, and its certificate flag.
   }
 }
 
