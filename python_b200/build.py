@@ -43,6 +43,18 @@ def build_engine(force: bool = False, verbose: bool = False) -> Path:
     return LIB
 
 
+def build_rounding_check(force: bool = False) -> Path:
+    """The kernel behind tests/test_gpu_rounding.py."""
+    lib, src = PKG / "_build" / "libcheck_rounding.so", CSRC / "check_rounding.cu"
+    if force or _stale(lib, [src, CSRC / "ss_common.cuh"]):
+        lib.parent.mkdir(exist_ok=True)
+        tmp = lib.with_suffix(".so.tmp")
+        subprocess.run([NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
+                        "-cudart", "static", "-o", str(tmp), str(src)], check=True, cwd=str(PKG))
+        os.replace(tmp, lib)
+    return lib
+
+
 def build_oracle(reference: bool = True) -> None:
     targets = ["port"]
     # the reference checkout: SIROCCO_REFERENCE, else a `reference` directory
