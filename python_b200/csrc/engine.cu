@@ -148,7 +148,7 @@ static KernelSpec small_spec(int cls, int mode) {
                ? reinterpret_cast<const void*>(&small_mixed_solve_kernel<NP, G>)        \
                : reinterpret_cast<const void*>(&small_exact_kernel<KIND, NP, G>);       \
     k.sys_per_block = kSmallThreads / G;                                                \
-    k.dyn_smem = small_smem_bytes<NP, G>();                                             \
+    k.dyn_smem = small_smem_bytes<KIND, NP, G>();                                       \
     break;
   switch (cls) {
 #include "small_classes.inc"

@@ -44,8 +44,6 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // barrier 1 over the first `count` threads (the panel warps)
 __device__ __forceinline__ void panel_bar(int count) { asm volatile("bar.sync 1, %0;\n" ::"r"(count) : "memory"); }
 
-constexpr int kSmemPerSm = 233472;   // shared memory of one SM (228 KB)
-
 // P: padded order; NT: threads; RG x CC: rows x columns of one update tile of
 // the workspace classes (columns tc + 8c; the shared-memory classes update one
 // column at a time); PW: panel warps; GM: matrix in a global workspace slab;

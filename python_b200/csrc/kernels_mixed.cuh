@@ -38,10 +38,20 @@ __device__ __forceinline__ double pow2_inv_scale(double m) {
   return ldexp(1.0, -e);
 }
 
+// CTAs per SM asked of the register allocator, which without a bound takes the
+// registers of one or two of them (order 16, 40,000 rate matrices: 437 us at 114
+// registers, 402 at 5 CTAs, 374 at 6; order 32, 4,096: 203 us at 164, 160 at 4).
+template <int NP>
+constexpr int mixed_min_blocks() {
+  return NP > 20 ? 4 : NP > 16 ? 5 : NP > 12 ? 6 : NP > 8 ? 7 : 8;
+}
+
 template <int NP, int G>
-__global__ void __launch_bounds__(kSmallThreads)
+__global__ void __launch_bounds__(kSmallThreads, (mixed_min_blocks<NP>()))
 small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
   constexpr int GPB = kSmallThreads / G;
+  static_assert(mixed_min_blocks<NP>() * (small_smem_bytes<kSolve, NP, G>() + 1024) <= kSmemPerSm,
+                "the CTAs asked for fit an SM");
   constexpr double kFloor = 1.0e-22;          // significance floor of a component (x_j / sum |x|)
   extern __shared__ __align__(16) unsigned char small_dsm[];
   SmallSmem<NP>* smem_all = reinterpret_cast<SmallSmem<NP>*>(small_dsm);   // [GPB]
@@ -50,15 +60,26 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
   const int lane = threadIdx.x % G;
   const unsigned gmask = group_mask<G>();
   SmallSmem<NP>& sm = smem_all[grp];
+  // over the space of the fallback's pivot rows: row and column scales, the
+  // broadcast pivot row, the row chosen at each step
+  double* rsc = sm.u;
+  double* csc = rsc + NP;
+  float* fpiv = reinterpret_cast<float*>(csc + NP);
+  int* lop = reinterpret_cast<int*>(fpiv + NP);
+  static_assert(2 * sizeof(double) + sizeof(float) + sizeof(int) <= sizeof(sm.u) / NP, "they fit");
 
+  // a warp's groups stay together, so that their fallbacks run together; a group
+  // past the list's end idles with n = 0
   const int count = batch_count(bv);
-  for (int item = blockIdx.x * GPB + grp; item < count; item += gridDim.x * GPB) {
-    const int s = bv.list[item];
-    const int n = bv.n[s];
-    const int64_t ov = bv.offv[s];
+  const int sub = (threadIdx.x & 31) / G;
+  for (int first = blockIdx.x * GPB + grp - sub; first < count; first += gridDim.x * GPB) {
+    const bool live = first + sub < count;
+    const int s = live ? bv.list[first + sub] : 0;
+    const int n = live ? bv.n[s] : 0;
+    const int64_t ov = live ? bv.offv[s] : 0;
     const double* __restrict__ bg = bv.b + ov;
     double* __restrict__ xg = bv.out + ov;
-    small_stage<NP, G>(sm, bv.A + bv.offA[s], n, lane, gmask);
+    small_stage<NP, G>(sm.stage, bv.A + (live ? bv.offA[s] : 0), n, lane, gmask);
     const bool act = lane < n;
     const int S = small_stride(n);
 
@@ -70,19 +91,19 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
         if (k < n) rmax = fmax(rmax, fabs(sm.stage[lane * S + k]));
     }
     const double rs = pow2_inv_scale(rmax);
-    if (act) sm.rsc[lane] = rs;
+    if (act) rsc[lane] = rs;
     __syncwarp(gmask);
     double cmax = 0.0;
     if (act) {
-      for (int r = 0; r < n; ++r) cmax = fmax(cmax, fabs(sm.stage[r * S + lane]) * sm.rsc[r]);
+      for (int r = 0; r < n; ++r) cmax = fmax(cmax, fabs(sm.stage[r * S + lane]) * rsc[r]);
     }
     const double cs_own = pow2_inv_scale(cmax);
-    if (act) sm.csc[lane] = cs_own;
+    if (act) csc[lane] = cs_own;
     __syncwarp(gmask);
     float af[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k)
-      af[k] = (act && k < n) ? float(sm.stage[lane * S + k] * rs * sm.csc[k]) : 0.0f;
+      af[k] = (act && k < n) ? float(sm.stage[lane * S + k] * rs * csc[k]) : 0.0f;
 
     // ---- 2. FP32 LU, rows stay in lanes; pstep = step that chose this row --
     bool done = false, bad = false;
@@ -111,16 +132,16 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
             done = true;
             pstep = j;
 #pragma unroll
-            for (int k = j; k < NP; ++k) sm.fpiv[k] = af[k];
+            for (int k = j; k < NP; ++k) fpiv[k] = af[k];
           }
           __syncwarp(gmask);
-          const float rinv = 1.0f / sm.fpiv[j];
+          const float rinv = 1.0f / fpiv[j];
           if (lane == kl) prinv = rinv;
           if (act && !was_done && lane != kl) {
             const float l = af[j] * rinv;
             af[j] = l;
 #pragma unroll
-            for (int k = j + 1; k < NP; ++k) af[k] = fmaf(-l, sm.fpiv[k], af[k]);
+            for (int k = j + 1; k < NP; ++k) af[k] = fmaf(-l, fpiv[k], af[k]);
           }
           __syncwarp(gmask);
         }
@@ -131,8 +152,8 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
     int diagbits = 0;
     if (bad || fallback) diagbits |= kDiagIllCond;
 
-    if (!fallback) {
-      if (act) sm.lop[pstep] = lane;
+    if (live && !fallback) {
+      if (act) lop[pstep] = lane;
       __syncwarp(gmask);
       // correction: returns, in lane j, the component j of C As^-1 R v
       auto correct = [&](double v) -> double {
@@ -145,7 +166,7 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
           if (j < n) {
-            const float yj = __shfl_sync(gmask, t, sm.lop[j], G);
+            const float yj = __shfl_sync(gmask, t, lop[j], G);
             if (act && pstep > j) t = fmaf(-af[j], yj, t);
           }
         }
@@ -154,12 +175,12 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
         for (int j = NP - 1; j >= 0; --j) {
           if (j < n) {
             const float zl = t * prinv;
-            const float zj = __shfl_sync(gmask, zl, sm.lop[j], G);
+            const float zj = __shfl_sync(gmask, zl, lop[j], G);
             if (act && pstep < j) t = fmaf(-af[j], zj, t);
             if (lane == j) dj = double(zj);
           }
         }
-        return act ? dj * sm.csc[lane] / sc : 0.0;
+        return act ? dj * csc[lane] / sc : 0.0;
       };
 
       double xj = correct(act ? bg[lane] : 0.0);
@@ -224,19 +245,22 @@ small_mixed_solve_kernel(BatchView bv, MixedParams mp) {
       }
     }
 
-    int code;
-    if (fallback) {
-      code = small_exact_solve<NP, G>(sm, act ? bg[lane] : 0.0, xg, n, lane, gmask);
-      diagbits |= kDiagFallback;
-    } else {
-      for (int k = lane; k < n; k += G) xg[k] = sm.xs[k];
-      code = kOk;
+    // the exact solve of the warp's systems that need it; the others idle in it
+    // (under each group's own mask its reductions run one group after another:
+    // 4,096 rate matrices of order 8: 39 us, 30 so; 40,000 of order 16: 374,
+    // 330 so)
+    int code = kOk;
+    if (__any_sync(0xffffffffu, fallback)) {
+      __syncwarp();
+      code = small_exact_solve<NP, G>(sm, act ? bg[lane] : 0.0, xg, fallback ? n : 0, lane, 0xffffffffu);
+      if (fallback) diagbits |= kDiagFallback;
     }
-    if (lane == 0) {
-      bv.status[s] = code;
+    if (!fallback && act) xg[lane] = sm.xs[lane];
+    if (live && lane == 0) {
+      bv.status[s] = fallback ? code : kOk;
       if (bv.diag) bv.diag[s] = diagbits | (iters & kDiagIterMask);
     }
-    __syncwarp(gmask);
+    __syncwarp();
   }
 }
 

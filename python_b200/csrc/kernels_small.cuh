@@ -17,24 +17,33 @@
 //          GSL's), above-pivot and already-inverted columns eliminated in the
 //          same sweep; columns are unscrambled in reverse pivot order at the end.
 #pragma once
+#include <type_traits>
+
 #include "ss_common.cuh"
 
 namespace ss {
 
 constexpr int kSmallThreads = 128;
 
+// A solve's shared memory (the mixed path keeps its scales in u, which only its
+// exact fallback needs for pivot rows).
 template <int NP>
 struct __align__(16) SmallSmem {
   static constexpr int S = NP + 1;   // odd row stride (in doubles) avoids bank conflicts
-  double stage[NP * S];              // A as loaded (solve: kept for the residual check); comes first
-  double u[NP * (NP + 3 - NP / 2)];  // the pivot rows by step (solve: small_urow; invert: the current one)
+  double stage[NP * S];              // A as loaded, kept for the residual check; comes first
+  double u[NP * (NP + 3 - NP / 2)];  // the pivot rows by step (small_urow)
   double xs[NP];                     // solution in natural order
-  float fpiv[NP];                    // broadcast pivot row (mixed path)
-  double rsc[NP];                    // row scales (mixed path)
-  double csc[NP];                    // column scales (mixed path)
+};
+
+// An inverse's: one pivot row at a time.  With a solve's pivot rows beside it fewer
+// CTAs fit an SM (20,000 inverses of order 32: 592 us, 390 so).
+template <int NP>
+struct __align__(16) SmallInvSmem {
+  static constexpr int S = NP + 1;
+  double stage[NP * S];              // A as loaded, then the rows of the result
+  double piv[NP];                    // broadcast pivot row
   int ipiv[NP];                      // position swapped with j at step j
-  int lop[NP];                       // lane holding position i (mixed path: the row chosen at step i)
-  int csrc[NP];                      // column unscramble map (invert)
+  int csrc[NP];                      // column unscramble map
 };
 
 // Start of pivot row j in SmallSmem::u: columns j & ~1 .. NP - 1, the row's
@@ -45,9 +54,9 @@ __host__ __device__ constexpr int small_urow(int j) {
 }
 
 // dynamic shared memory of a launch
-template <int NP, int G>
+template <int KIND, int NP, int G>
 constexpr size_t small_smem_bytes() {
-  return sizeof(SmallSmem<NP>) * (kSmallThreads / G);
+  return (KIND == kSolve ? sizeof(SmallSmem<NP>) : sizeof(SmallInvSmem<NP>)) * (kSmallThreads / G);
 }
 
 template <int G>
@@ -60,13 +69,12 @@ __device__ __forceinline__ unsigned group_mask() {
 // read by rows falls on distinct banks.
 __device__ __forceinline__ int small_stride(int n) { return n | 1; }
 
-// Coalesced load of a system into sm.stage (rows small_stride(n) apart), every
+// Coalesced load of a system into `stage` (rows small_stride(n) apart), every
 // load of the lane issued before the first shared-memory store so they are all
 // in flight together.  Element e = r n + c goes to e + r for an even n; e / n by
 // a 16-bit reciprocal, exact for e < 1024, n <= 32.
 template <int NP, int G>
-__device__ __forceinline__ void small_stage(SmallSmem<NP>& sm, const double* __restrict__ Ag, int n, int lane,
-                                            unsigned gmask) {
+__device__ __forceinline__ void small_stage(double* stage, const double* __restrict__ Ag, int n, int lane, unsigned gmask) {
   constexpr int PER = (NP * NP + G - 1) / G;
   const int nn = n * n;
   double v[PER];
@@ -80,7 +88,7 @@ __device__ __forceinline__ void small_stage(SmallSmem<NP>& sm, const double* __r
 #pragma unroll
   for (int u = 0; u < PER; ++u) {
     const unsigned e = unsigned(lane + u * G);
-    if (int(e) < nn) sm.stage[e + even * ((e * inv) >> 16)] = v[u];
+    if (int(e) < nn) stage[e + even * ((e * inv) >> 16)] = v[u];
   }
   __syncwarp(gmask);
 }
@@ -88,14 +96,14 @@ __device__ __forceinline__ void small_stage(SmallSmem<NP>& sm, const double* __r
 // GSL-exact Gauss-Jordan sweep of the row held in a[].  Returns true when U has
 // an exact zero on its diagonal.
 template <int NP, int G>
-__device__ __forceinline__ bool small_exact_gj(SmallSmem<NP>& sm, double (&a)[NP], int n, int lane,
+__device__ __forceinline__ bool small_exact_gj(SmallInvSmem<NP>& sm, double (&a)[NP], int n, int lane,
                                                unsigned gmask, int& pos, bool& inf_piv) {
   const bool act = lane < n;
   bool done = false;
   bool sing = false;
   inf_piv = false;
   pos = lane;
-  double* piv = sm.u;
+  double* piv = sm.piv;
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
     if (j < n && !sing) {
@@ -407,12 +415,15 @@ __device__ __forceinline__ int small_exact_solve(SmallSmem<NP>& sm, double bi, d
   return sing ? kSolveSingular : code;
 }
 
-// CTAs per SM asked of the register allocator for a solve: as many as fit
-// without spilling the row (measured with one more or less: NP = 28 47.2 us at
-// 4, 48.7 at 5; 16 97.0 at 5, 99.7 at 4; 12 61.4 at 6, 64.6 at 5).
+// CTAs per SM asked of the register allocator.  Solves: the best of those measured
+// (NP = 28 47.2 us at 4, 48.7 at 5; 16 97.0 at 5, 99.7 at 4; 12 61.4 at 6, 64.6 at
+// 5); no row is spilled but at NP = 24, 44 bytes at 5.  Inverses: as many as hold
+// their rows without spilling; left to itself the allocator takes up to 186
+// registers (20,000 of order 16: 104 us at 102 registers, 82 at 80).
 template <int KIND, int NP>
 constexpr int small_min_blocks() {
-  return KIND != kSolve ? 1 : NP > 28 ? 3 : NP > 24 ? 4 : NP > 12 ? 5 : 6;
+  if (KIND != kSolve) return NP > 20 ? 4 : NP > 16 ? 5 : NP > 12 ? 6 : NP > 8 ? 7 : NP > 4 ? 8 : 9;
+  return NP > 28 ? 3 : NP > 24 ? 4 : NP > 12 ? 5 : 6;
 }
 
 template <int KIND, int NP, int G>
@@ -420,14 +431,15 @@ __global__ void __launch_bounds__(kSmallThreads, (small_min_blocks<KIND, NP>()))
 small_exact_kernel(BatchView bv) {
   static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group size");
   static_assert(NP <= G, "one row per lane");
+  static_assert(small_min_blocks<KIND, NP>() * (small_smem_bytes<KIND, NP, G>() + 1024) <= kSmemPerSm,
+                "the CTAs asked for fit an SM");
   constexpr int GPB = kSmallThreads / G;       // groups per block
-  constexpr int S = SmallSmem<NP>::S;
   extern __shared__ __align__(16) unsigned char small_dsm[];
-  SmallSmem<NP>* smem_all = reinterpret_cast<SmallSmem<NP>*>(small_dsm);   // [GPB]
+  using Smem = std::conditional_t<KIND == kSolve, SmallSmem<NP>, SmallInvSmem<NP>>;
 
   const int grp = threadIdx.x / G;
   const int lane = threadIdx.x % G;
-  SmallSmem<NP>& sm = smem_all[grp];
+  Smem& sm = reinterpret_cast<Smem*>(small_dsm)[grp];   // [GPB]
   const int count = batch_count(bv);
 
   if constexpr (KIND == kSolve) {
@@ -446,7 +458,7 @@ small_exact_kernel(BatchView bv) {
     for (; first < count; first += stride) {
       const int s2 = system(first + stride + sub);
       const double bi = (lane < n) ? bv.b[ov + lane] : 0.0;
-      small_stage<NP, G>(sm, bv.A + oa, n, lane, 0xffffffffu);
+      small_stage<NP, G>(sm.stage, bv.A + oa, n, lane, 0xffffffffu);
       const int n2 = s2 >= 0 ? bv.n[s2] : 0;
       const int64_t oa2 = s2 >= 0 ? bv.offA[s2] : 0, ov2 = s2 >= 0 ? bv.offv[s2] : 0;
       const int code = small_exact_solve<NP, G>(sm, bi, bv.out + ov, n, lane, 0xffffffffu);
@@ -462,14 +474,13 @@ small_exact_kernel(BatchView bv) {
       oa = oa2;
       ov = ov2;
     }
-    return;
-  }
-  const unsigned gmask = group_mask<G>();
-  for (int item = blockIdx.x * GPB + grp; item < count; item += gridDim.x * GPB) {
-    const int s = bv.list[item];
-    const int n = bv.n[s];
-    small_stage<NP, G>(sm, bv.A + bv.offA[s], n, lane, gmask);
-    {
+  } else {
+    constexpr int S = SmallInvSmem<NP>::S;
+    const unsigned gmask = group_mask<G>();
+    for (int item = blockIdx.x * GPB + grp; item < count; item += gridDim.x * GPB) {
+      const int s = bv.list[item];
+      const int n = bv.n[s];
+      small_stage<NP, G>(sm.stage, bv.A + bv.offA[s], n, lane, gmask);
       const bool act = lane < n;
       double a[NP];
 #pragma unroll
@@ -509,8 +520,8 @@ small_exact_kernel(BatchView bv) {
         bv.status[s] = code;
         if (bv.diag) bv.diag[s] = kDiagExact;
       }
+      __syncwarp(gmask);
     }
-    __syncwarp(gmask);
   }
 }
 

@@ -82,6 +82,8 @@ struct MixedParams {
   double resid_margin;    // residual-check value above which exact FP64 decides the code
 };
 
+constexpr int kSmemPerSm = 233472;   // shared memory of one SM (228 KB)
+
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }

@@ -19,7 +19,7 @@ struct Candidate {
 };
 
 #define SS_TUNE_SMALL(NP, G) \
-  {NP, G, reinterpret_cast<const void*>(&ss::small_exact_kernel<ss::kSolve, NP, G>), ss::small_smem_bytes<NP, G>()},
+  {NP, G, reinterpret_cast<const void*>(&ss::small_exact_kernel<ss::kSolve, NP, G>), ss::small_smem_bytes<ss::kSolve, NP, G>()},
 const Candidate kCand[] = {
 #include "tune_small_candidates.inc"
 };
