@@ -289,7 +289,7 @@ struct Bucket {
   int phase;      // 1: certified kernels and directly listed systems; 2: fallback lists
   int fb;         // phase 2: index of the fallback list this launch serves
   int q;          // streamed certified inverses: index of the launch's queue counter
-  bool fills;     // small systems that fill the GPU at least twice over
+  bool fills;     // exact small solves that fill the GPU at least twice over
 };
 
 }  // namespace ss
@@ -521,7 +521,7 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
     if (rc) return rc;
     const int blocks_needed = (b.count + b.spec.sys_per_block - 1) / b.spec.sys_per_block;
     b.grid = std::max(1, std::min(blocks_needed * b.spec.cluster, b.spec.max_ctas));
-    b.fills = fam == kFamSmall && fb < 0 && blocks_needed >= 2 * b.spec.max_ctas;
+    b.fills = fam == kFamSmall && kind == kSolve && mode != SIROCCO_MIXED && blocks_needed >= 2 * b.spec.max_ctas;
     if (fam == kFamGlobal && kind == kSolve) {
       b.slab = (int64_t(cls) * cls + 31) / 32 * 32;
       b.scratch_off = scratch_elems;
@@ -664,10 +664,12 @@ static int launch_bucket(const sirocco_plan* p, const Bucket& b, const double* A
 }
 
 // The buckets of one phase, forked onto the side streams and joined back into
-// st.  Small-system buckets that fill the GPU on their own run one after another
-// instead: their kernels are unrolled over the order, and two of them on one SM
-// evict each other's code from the instruction cache (200,000 systems of orders
-// 2-27: 522 us forked, 506 us in turn).
+// st.  Exact small solves whose buckets fill the GPU on their own run one after
+// another instead: their kernels are unrolled over the order, and two of them on
+// one SM evict each other's code from the instruction cache (200,000 systems of
+// orders 2-27: 522 us forked, 506 us in turn).  Inverses and mixed solves are
+// better forked (60,000 systems of orders 2-32: 457 us against 486 in turn, and
+// 568 against 604).
 static int run_phase(sirocco_plan* p, int phase, const double* A, const double* bvec, double* out, int* status,
                      int* diag, cudaStream_t st) {
   std::vector<const Bucket*> bs, queue;   // queue: one after another on st
