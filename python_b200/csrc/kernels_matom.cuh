@@ -150,6 +150,12 @@ __global__ void __launch_bounds__(128) matom_epilogue_tile_kernel(int nsys, cons
 // Four draws to a warp, each to its end, took 282 us: most loads were then those
 // of the longest walk.)
 constexpr int kDrawThreads = 256, kDrawSlots = 4, kDrawBlocksPerSM = 7;
+// Rows that one round covers cost the warp a whole round each; where many of a
+// warp's draws have such rows, each is walked by the lane of its draw instead, all
+// of them together (4 million draws from rows of 4: 228 us by rounds, 64 walked; of
+// 10: 220, 87; of 30: 220, 181; of 32: 222, 270).  With few of them the walk, one load
+// at a time, would hold up the warp's other draws (orders 20-200: 125 us against 122).
+constexpr int kDrawShort = 31, kDrawShortLanes = 8;
 
 // Draws per warp: 32, or fewer where that would leave warps of the GPU without
 // any, but one for every slot.
@@ -181,6 +187,16 @@ matom_sample_kernel(int nq, int per, int nsys, const int* __restrict__ n, const 
         nl = (0.0 < zl) ? ns : 0;
       }
     }
+  }
+  // rows shorter than a round are walked by their draws' own lanes, together
+  const unsigned brief = __ballot_sync(0xffffffffu, nl > 0 && nl <= kDrawShort);
+  if (__popc(brief) >= kDrawShortLanes && (brief >> lane & 1u)) {
+    for (int c = 0; c < nl; ++c)
+      if (!(__ldg(C + off + c) < zl)) {
+        ans = c;
+        break;
+      }
+    nl = 0;
   }
   unsigned todo = __ballot_sync(0xffffffffu, nl > 0);
   const double* row[kDrawSlots];   // the next totals of each slot's draw
