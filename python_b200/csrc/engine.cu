@@ -67,7 +67,8 @@ enum Family : int { kFamSmall = 0, kFamCta = 1, kFamGlobal = 2, kFamCgj = 3, kFa
 
 struct KernelSpec {
   const void* fn = nullptr;
-  const void* fn_epi = nullptr;   // certified family: the kernel with the macro-atom epilogue
+  const void* fn_b = nullptr;     // certified family: the kernels that write B, and B and C
+  const void* fn_bc = nullptr;
   int threads = 0;
   size_t dyn_smem = 0;
   int sys_per_block = 1;
@@ -200,7 +201,8 @@ static KernelSpec cgj_spec(int cls) {
   case I: {                                                                              \
     using Sh = CgjShape<P, WGR, WGC, CL, MINB, ST>;                                      \
     k.fn = reinterpret_cast<const void*>(&cgj_inverse_kernel<P, WGR, WGC, CL, MINB, ST>); \
-    k.fn_epi = reinterpret_cast<const void*>(&cgj_inverse_kernel<P, WGR, WGC, CL, MINB, ST, true>); \
+    k.fn_b = reinterpret_cast<const void*>(&cgj_inverse_kernel<P, WGR, WGC, CL, MINB, ST, kCertB>); \
+    k.fn_bc = reinterpret_cast<const void*>(&cgj_inverse_kernel<P, WGR, WGC, CL, MINB, ST, kCertTotals>); \
     k.threads = Sh::NTH;                                                             \
     k.dyn_smem = Sh::dyn_smem;                                                       \
     k.cluster = CL;                                                                  \
@@ -238,7 +240,7 @@ static int finish_spec(KernelSpec& k) {
     set_error("no kernel for this size class");
     return SIROCCO_ESIZE;
   }
-  for (const void* f : {k.fn, k.fn_epi})
+  for (const void* f : {k.fn, k.fn_b, k.fn_bc})
     if (f && k.dyn_smem > 0)
       SS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.dyn_smem)));
   int nb = 0;
@@ -641,7 +643,7 @@ static int launch_bucket(const sirocco_plan* p, const Bucket& b, const double* A
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = b.spec.cluster > 1 ? 1 : 0;
-    SS_CUDA(cudaLaunchKernelExC(&cfg, (ep.R || ep.C) ? b.spec.fn_epi : b.spec.fn, args));
+    SS_CUDA(cudaLaunchKernelExC(&cfg, ep.C ? b.spec.fn_bc : ep.R ? b.spec.fn_b : b.spec.fn, args));
   } else if (b.fam == kFamGlobal) {
     int nmax = b.cls;
     double* scratch = p->d_scratch ? p->d_scratch + b.scratch_off : nullptr;

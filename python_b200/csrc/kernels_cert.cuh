@@ -364,9 +364,13 @@ __device__ __forceinline__ void warp_inv8_refined(double& d0, double& d1, int la
   }
 }
 
-// EPI: the macro-atom epilogue is compiled in (CertEpi); without it the kernel
-// writes the inverse and its registers are the factorisation's alone.
-template <int P, int WGR, int WGC, int CL, int MINB, bool STAGE = true, bool EPI = false>
+// What the kernel writes (CertEpi): the inverse, B, or B and its running totals.  Each
+// is a kernel of its own: the totals' code takes registers from the factorisation
+// (1,500 cells of order 200, B alone: 2,016 us by the totals' kernel, 1,919 by
+// B's; of 144: 758, 697; of 104: 288, 312).
+enum CertOut : int { kCertInverse = 0, kCertB = 1, kCertTotals = 2 };
+
+template <int P, int WGR, int WGC, int CL, int MINB, bool STAGE = true, int OUT = kCertInverse>
 __global__ void __launch_bounds__(32 * WGR * WGC + 32, MINB)
 cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
   using S = CgjShape<P, WGR, WGC, CL, MINB, STAGE>;
@@ -848,7 +852,7 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
     // and wait for one another after them: a release behind the stores would
     // hold every warp until they have all landed.
     cluster_arrive<CL>();
-    if (EPI && ep.R && tile) {
+    if (OUT != kCertInverse && tile) {
       const double* __restrict__ Rs = ep.R + ep.offv[s];
 #pragma unroll
       for (int j = 0; j < WC; ++j)
@@ -877,7 +881,7 @@ cgj_inverse_kernel(BatchView bv, CertArgs ca, CertEpi ep) {
       }
     }
     cluster_wait<CL>();
-    if (EPI && ep.C) {
+    if (OUT == kCertTotals) {
       // Running totals of each row this CTA holds, left to right as the reference
       // adds them, 16 columns at a time through shared memory (the panel buffers,
       // free now).  Three pieces are under way: the warps that hold
