@@ -746,8 +746,8 @@ struct PinBuf {
     if (want <= bytes) return 0;
     release();
     SS_CUDA(cudaHostAlloc(&ptr, want, cudaHostAllocMapped));
-    bytes = want;
     SS_CUDA(cudaHostGetDevicePointer(&dev, ptr, 0));
+    bytes = want;
     return 0;
   }
   void release() {
@@ -979,6 +979,16 @@ static bool is_device_ptr(const void* ptr) {
     return false;
   }
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
+}
+
+// false for memory of a GPU that host code must not touch (managed memory it may)
+static bool host_can_reach(const void* ptr) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return at.type != cudaMemoryTypeDevice;
 }
 
 static int run_batched(int kind, int nsys, const int* n, const int64_t* offA, const double* A,
@@ -1983,7 +1993,8 @@ static int run_macro_pops(int ncell, int n, int nion, const int* ion_first, cons
 }
 
 // page-locked memory a thread's drop-in calls may hold (an inverse of order 361);
-// larger systems, whose kernels take milliseconds, go through pageable copies
+// larger systems, whose kernels take milliseconds, go through pageable copies, and
+// so do buffers in device memory, which the copies take as well
 constexpr size_t kMaxPinBytes = size_t(2) << 20, kMinPinBytes = size_t(64) << 10;
 
 static int run_single_pageable(Context* c, sirocco_plan* p, int kind, const double* A, const double* b, int size,
@@ -2031,8 +2042,13 @@ static int run_single(int kind, double* A, const double* b, int size, double* ou
   // waited for by itself: 64 us a solve of order 27, with the same kernel 56 us;
   // 34 us now.)
   const size_t total = sizeof(double) * (nA + nV + nO + 1);
-  if (total > kMaxPinBytes) return run_single_pageable(c, p, kind, A, b, size, out, code);
-  if ((rc = c->pin.ensure(std::max(total, kMinPinBytes)))) return rc;
+  if (total > kMaxPinBytes || !host_can_reach(A) || (kind == kSolve && !host_can_reach(b)) || !host_can_reach(out))
+    return run_single_pageable(c, p, kind, A, b, size, out, code);
+  // no page-locked memory to be had: the pageable way needs none
+  if (c->pin.ensure(std::max(total, kMinPinBytes))) {
+    cudaGetLastError();
+    return run_single_pageable(c, p, kind, A, b, size, out, code);
+  }
   double* h = static_cast<double*>(c->pin.ptr);
   double* hout = h + nA + nV;
   int* hcode = reinterpret_cast<int*>(hout + nO);
