@@ -385,6 +385,14 @@ static int check_layout(int kind, int nsys, const int* n, const int64_t* offA, c
   return 0;
 }
 
+// A copy from pageable memory may return before it has landed, and a memset does;
+// both run on the default stream, for which the streams that read their results
+// (non-blocking ones, here and often the caller's) do not wait.
+static int default_stream_done() {
+  SS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return 0;
+}
+
 static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, const int64_t* offA,
                       const int64_t* offv, int mode, bool alloc_scratch = true) {
   *out = nullptr;
@@ -600,6 +608,7 @@ static int plan_build(sirocco_plan** out, int kind, int nsys, const int* n, cons
     p->ev.push_back(e);
   }
   SS_CUDA(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
+  if (int rc2 = default_stream_done()) return rc2;
   *out = p.release();
   return 0;
 }
@@ -1515,6 +1524,7 @@ static int ion_asm_prepare(const sirocco_ion_table* t, int ncell, const sirocco_
     if (dsz[k] > 0) SS_CUDA(cudaMemcpy(dd + off, dsrc[k], sizeof(double) * dsz[k], cudaMemcpyHostToDevice));
     off += dsz[k];
   }
+  if ((rc = default_stream_done())) return rc;
   v = IonAsmView{};
   v.nions = nions;
   v.nelem = nelem;
@@ -1839,6 +1849,7 @@ static int run_matom_rate_matrices(const sirocco_matom_table* t, int ncell, cons
     if (dsz[k] > 0) SS_CUDA(cudaMemcpy(dd + off, dsrc[k], sizeof(double) * dsz[k], cudaMemcpyHostToDevice));
     off += dsz[k];
   }
+  if ((rc = default_stream_done())) return rc;
   MatomAsmView v{};
   v.nlev = nlev;
   v.n_bbd = n_bbd;
