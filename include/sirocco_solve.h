@@ -89,7 +89,8 @@ int gpu_invert_matrix(double *matrix, double *inverse, int num_rows);
    (element offset of each right-hand side in b and solution in x) are HOST
    arrays; A, b, x and status may all be host or all be device pointers.
    Returns 0, a negative library code, or a CUDA error code; status[s] holds the
-   reference code of system s.  For a singular system x is left unspecified. */
+   reference code of system s.  For a singular system x is left unspecified.  x may
+   be the same buffer as b. */
 int solve_matrix_batched(int nsys, const int *n, const int64_t *offA, const double *A,
                          const int64_t *offv, const double *b, double *x, int *status);
 

@@ -1,5 +1,5 @@
-// CTA-per-system kernels for 32 < n <= 256 (macro-atom jumping matrices of a
-// few dozen to a few hundred levels, per-element macro populations).
+// CTA-per-system kernels for 32 < n <= 1024 (macro-atom jumping matrices of a few
+// dozen levels and more, per-element macro populations).
 //
 // The padded P x P matrix is held row-major with its columns XOR-swizzled
 // inside 16-column groups (row, column and tile accesses are then free of
@@ -277,7 +277,7 @@ cta_exact_kernel(BatchView bv, double* __restrict__ work) {
               for (int i = 1; i < RPL; ++i) mine = (pi == i) ? pr[i][c] : mine;
               pv[c] = __shfl_sync(FULL, mine, pl);
             }
-            rinv = __shfl_sync(FULL, rb, pl);   // = fl(1/u_jj), correctly rounded
+            rinv = __shfl_sync(FULL, rb, pl);   // = fl(1/u_jj) where rcp_covers(u_jj)
           }
           const double ujj = pv[0];
           if (!rcp_covers(ujj)) rinv = rcp_outline(ujj);   // the same on every lane

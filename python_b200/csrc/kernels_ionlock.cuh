@@ -9,7 +9,7 @@
 // populations leaves the SM, and the host takes part only before and after.
 // What bounds it is the chain of the largest element's solve, once per round,
 // times the rounds of the cell that takes the most.  4,096 cells of five elements
-// took 21.1 ms a call with rounds driven by the host (a layout, a plan, five
+// took 21.5 ms a call with rounds driven by the host (a layout, a plan, five
 // launches and four copies each); now 4.9 ms, of which 3 are the 200 rounds of a
 // cell that never converges (15 us each) and about 1.5 the copies in and out.
 #pragma once
