@@ -1515,16 +1515,17 @@ static int ion_asm_prepare(const sirocco_ion_table* t, int ncell, const sirocco_
     return rc;
   int* di_ = static_cast<int*>(c->bIT.ptr);
   double* dd = static_cast<double*>(c->bID.ptr);
-  SS_CUDA(cudaMemcpy(di_, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice));
-  SS_CUDA(cudaMemcpy(c->bI64.ptr, boff.data(), sizeof(int64_t) * nelem, cudaMemcpyHostToDevice));
+  // on the stream that reads them; pageable sources are free again when a copy returns
+  SS_CUDA(cudaMemcpyAsync(di_, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice, c->stream));
+  SS_CUDA(cudaMemcpyAsync(c->bI64.ptr, boff.data(), sizeof(int64_t) * nelem, cudaMemcpyHostToDevice, c->stream));
   const double* dptr[9];
   size_t off = 0;
   for (int k = 0; k < 9; ++k) {
     dptr[k] = dd + off;
-    if (dsz[k] > 0) SS_CUDA(cudaMemcpy(dd + off, dsrc[k], sizeof(double) * dsz[k], cudaMemcpyHostToDevice));
+    if (dsz[k] > 0)
+      SS_CUDA(cudaMemcpyAsync(dd + off, dsrc[k], sizeof(double) * dsz[k], cudaMemcpyHostToDevice, c->stream));
     off += dsz[k];
   }
-  if ((rc = default_stream_done())) return rc;
   v = IonAsmView{};
   v.nions = nions;
   v.nelem = nelem;
@@ -1841,15 +1842,16 @@ static int run_matom_rate_matrices(const sirocco_matom_table* t, int ncell, cons
     return rc;
   int* di_ = static_cast<int*>(c->bMT.ptr);
   double* dd = static_cast<double*>(c->bMD.ptr);
-  SS_CUDA(cudaMemcpy(di_, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice));
+  // on the stream that reads them; pageable sources are free again when a copy returns
+  SS_CUDA(cudaMemcpyAsync(di_, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice, c->stream));
   const double* dp[ND];
   size_t off = 0;
   for (int k = 0; k < ND; ++k) {
     dp[k] = dd + off;
-    if (dsz[k] > 0) SS_CUDA(cudaMemcpy(dd + off, dsrc[k], sizeof(double) * dsz[k], cudaMemcpyHostToDevice));
+    if (dsz[k] > 0)
+      SS_CUDA(cudaMemcpyAsync(dd + off, dsrc[k], sizeof(double) * dsz[k], cudaMemcpyHostToDevice, c->stream));
     off += dsz[k];
   }
-  if ((rc = default_stream_done())) return rc;
   MatomAsmView v{};
   v.nlev = nlev;
   v.n_bbd = n_bbd;
